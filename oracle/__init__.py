@@ -58,8 +58,11 @@ def build_oracle() -> None:
 
 def reference_root() -> str:
     """Root of the reference source tree: $AW_REFERENCE_ROOT when set, else
-    the read-only checkout this build was developed against."""
-    return os.environ.get("AW_REFERENCE_ROOT", "/root/reference")
+    the read-only checkout this build was developed against. An empty
+    directory (a mount point without the tree) is answered with the path of a
+    part of the tree that is missing, so that it counts as absent."""
+    root = os.environ.get("AW_REFERENCE_ROOT", "/root/reference")
+    return os.path.join(root, "Code") if os.path.isdir(root) and not os.listdir(root) else root
 
 
 def build_reference(ref_root: Optional[str] = None) -> bool:

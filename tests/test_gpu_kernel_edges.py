@@ -1,0 +1,141 @@
+"""The kernels at the sizes and inputs where their paths change, against the
+oracle.
+
+* The in-place transforms of the any-size fluid operator: the smallest axes,
+  odd rows and slabs (a row pair without its second row), primes above the
+  register radices, one to four stages an axis, extra places of the packed
+  column on one line (ny = 2), slabs beyond one block. The bound is that of
+  the operator's other tests, 1e-5 of max |fp64|; a transform of n values
+  rounds each of them about 3 log2(n) times to 6e-8, under 4e-6 for three
+  axes of 512.
+* The splat's sums: destinations whose candidates come in order, out of
+  order, more than fit the list, buckets left unsorted and sorted. Bit-exact.
+* The direct kernel's data gradient, with one, two and four planes a tile and
+  with and without the ReLU mask: BF16 outputs to 1e-2 of max |ref|, the
+  bound of the GEMM path's test (one BF16 rounding is 2^-9).
+* Interpolation at the volume's borders, at positions just below zero (whose
+  fraction is not a float), at integers, and beyond the range of the fast
+  floor. Bit-exact.
+"""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from atlaswerks_b200 import _lib  # noqa: E402
+from atlaswerks_b200 import device as D  # noqa: E402
+from atlaswerks_b200.greedy import DiffOperB200, DiffOperParam  # noqa: E402
+from oracle import identity  # noqa: E402
+from oracle import nn_oracle as O  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def cu(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def host(t):
+    torch.cuda.synchronize()
+    return t.cpu().numpy()
+
+
+@pytest.mark.parametrize("shape", [
+    (2, 2, 2), (2, 2, 3), (3, 2, 2), (2, 3, 2), (3, 3, 3), (2, 4, 6),  # [nz, ny, nx]
+    (5, 7, 9), (11, 13, 10), (13, 12, 11),
+    (17, 18, 16), (16, 17, 34), (19, 16, 23), (7, 62, 31), (109, 4, 6), (6, 109, 38), (8, 6, 181),
+    (289, 3, 4), (3, 4, 289),                                          # two primes above the radices
+    (96, 20, 24), (20, 243, 12), (250, 6, 10), (512, 6, 4), (4, 512, 6), (4, 6, 509),
+    (3, 330, 257), (4, 299, 300)])
+@pytest.mark.parametrize("inverse", [True, False])
+def test_fluid_operator_any_axis(oracle, shape, inverse):
+    rng = np.random.default_rng(31)
+    sp = (1.0, 1.3, 0.8)
+    f = rng.normal(0, 1, (3,) + shape).astype(np.float32)
+    want = oracle.fluid_f64(f, sp, inverse=inverse)
+    op = DiffOperB200()
+    op.SetSize(shape[::-1], sp, DiffOperParam())
+    v = cu(f)
+    (op.ApplyInverseOperator if inverse else op.ApplyOperator)(v)
+    err = np.abs(host(v).astype(np.float64) - want).max() / np.abs(want).max()
+    assert err <= 1e-5, err
+    assert not op.TimedOut()
+
+
+@pytest.mark.parametrize("shape", [(12, 11, 10), (9, 17, 131), (20, 18, 16)])
+@pytest.mark.parametrize("scale", [1.0, 0.85, 0.7, 0.55, 0.42, 0.3])
+@pytest.mark.parametrize("jitter", [0.0, 0.3])
+def test_splat_candidate_counts(oracle, shape, scale, jitter):
+    """scale^-3 sources a cell: 1, 1.6, 2.9, 6, 13, 37; eight times that per destination."""
+    rng = np.random.default_rng(32)
+    img = rng.normal(0, 1, shape).astype(np.float32)
+    h = identity(shape) * np.float32(scale) + rng.normal(0, 1, (3,) + shape) * jitter + 0.3
+    h = h.astype(np.float32)
+    want = oracle.splat(img, h, 0.25)
+    for _ in range(2):  # the arrival order inside a bucket may differ
+        assert np.array_equal(host(D.splat(cu(img), cu(h), 0.25)), want)
+
+
+@pytest.mark.parametrize("grid", [(1, 8, 32, 16), (2, 6, 32, 24), (1, 3, 32, 16), (1, 32, 64, 64)])
+@pytest.mark.parametrize("cin,cout", [(16, 16), (48, 16), (16, 32), (32, 32)])
+@pytest.mark.parametrize("masked", [True, False])
+def test_conv_dgrad_direct(grid, cin, cout, masked):
+    B, DD, H, W = grid
+    rng = np.random.default_rng(36)
+    dy = O.bf16(rng.normal(0, 1, grid + (cout,)).astype(np.float32))
+    w = O.bf16(rng.normal(0, 0.1, (cout, 27, cin)).astype(np.float32))
+    mask = O.bf16(rng.normal(0, 1, grid + (cin,)).astype(np.float32)) if masked else None
+    want = O.conv_dgrad(dy, w, mask if masked else np.ones(grid + (cin,), np.float32))
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(torch.bfloat16).cuda()  # noqa: E731
+    dyd, wtd, md = dev(dy), dev(w.transpose(2, 1, 0)), dev(mask) if masked else None
+    dx = torch.zeros((B * DD * H * W, cin), dtype=torch.bfloat16, device="cuda")
+    rc = _lib.lib().aw_nn_conv3d_dgrad(dyd.data_ptr(), B, DD, H, W, cout, wtd.data_ptr(), cin, 27,
+                                       md.data_ptr() if masked else None, dx.data_ptr(), None, 0, None)
+    assert rc == 0, _lib.lib().aw_last_error()
+    got = host(dx.float()).reshape(want.shape)
+    assert np.abs(got - want).max() <= 1e-2 * np.abs(want).max()
+
+
+def _edge_field(shape, rng):
+    """Positions all over the borders, a tenth of them special."""
+    h = identity(shape) + rng.normal(0, 0.6, (3,) + shape).astype(np.float32)
+    special = np.float32([0.0, -0.0, -1e-10, -1e-30, 1e-10, -0.5, 0.5, 1.0, -1.0, 2.0 ** 21, -2.0 ** 21,
+                          2.0 ** 22 + 1, 2.0 ** 23 - 1, -2.0 ** 23 - 1, 1e9])
+    pick = rng.random(h.shape) < 0.1
+    h[pick] = special[rng.integers(0, special.size, int(pick.sum()))]
+    for a in range(3):  # the far border too
+        n = shape[2 - a]
+        far = rng.random(h[a].shape) < 0.05
+        h[a][far] = (n - 1) + rng.choice(np.float32([0.0, -1e-6, 1e-6, 0.5, 1.0]), int(far.sum()))
+    return h.astype(np.float32)
+
+
+@pytest.mark.parametrize("shape", [(8, 9, 33), (5, 4, 130), (2, 2, 2)])
+def test_apply_at_the_edges(oracle, shape):
+    rng = np.random.default_rng(33)
+    img = rng.random(shape, dtype=np.float32)
+    h = _edge_field(shape, rng)
+    assert np.array_equal(host(D.apply(cu(img), cu(h), 0.7)), oracle.apply(img, h, 0.7))
+
+
+@pytest.mark.parametrize("shape", [(8, 9, 33), (2, 2, 2)])
+@pytest.mark.parametrize("bg", range(4))
+@pytest.mark.parametrize("sp", [(1.0, 1.0, 1.0), (1.5, 0.75, 1.2)])
+def test_compose_at_the_edges(oracle, shape, bg, sp):
+    rng = np.random.default_rng(34)
+    g = identity(shape) + rng.normal(0, 1, (3,) + shape).astype(np.float32)
+    v = rng.normal(0, 1, (3,) + shape).astype(np.float32)
+    h = _edge_field(shape, rng)
+    got = host(D.compose_vh(cu(v), cu(h), sp, 1.0, -1, bg))
+    assert np.array_equal(got, oracle.compose_vh(v, h, sp, -1, bg))
+    u = ((h - identity(shape)) * np.float32(sp).reshape(3, 1, 1, 1)).astype(np.float32)
+    got = host(D.compose_hv(cu(g), cu(u), sp, 1.0, 1, bg))
+    assert np.array_equal(got, oracle.compose_hv(g, u, sp, 1, bg))
+
+
+@pytest.mark.parametrize("sp", [(1.5, 0.75, 1.25), (1.2, 0.9, 2.06452), (2.0, 0.5, 1.0)])
+def test_gradient_divisors(oracle, sp):
+    """Spacings divided in float (exactly floats), in double, and multiplied."""
+    rng = np.random.default_rng(35)
+    img = rng.normal(0, 1, (7, 9, 12)).astype(np.float32)
+    assert np.array_equal(host(D.gradient(cu(img), sp)), oracle.gradient(img, sp, False))
