@@ -60,9 +60,16 @@ AW_D float fdiv(float a, float b) { return __fdiv_rn(a, b); }
 // x / d as the reference divides (IEEE, round to nearest). When d is a power
 // of two the quotient is x scaled by an exact power of two, and x * (1/d)
 // is the same number: the multiply replaces the division sequence.
+// A float x divided in double and rounded to float is also one float
+// operation where the divisor allows it (div_float): x / d in float when d is
+// a float (the double quotient of two floats never rounds onto a float
+// midpoint it was not on: 53 >= 2 * 24 + 2, Figueroa 1995), x * (1/d) when d
+// is a power of two whose reciprocal is a normal float.
 struct DivD {
   double d, r;
   int p2;
+  int as;        // div_float: 2 multiply by fr, 1 divide by fd, 0 in double
+  float fd, fr;
 };
 struct DivF {
   float d, r;
@@ -74,9 +81,21 @@ inline bool host_is_pow2(double d) {
   const double m = frexp(d, &e);
   return m == 0.5 && e > -1000 && e < 1000;
 }
-inline DivD make_div(double d) { return DivD{d, 1.0 / d, host_is_pow2(d) ? 1 : 0}; }
+inline DivD make_div(double d) {
+  DivD q{d, 1.0 / d, host_is_pow2(d) ? 1 : 0, 0, (float)d, (float)(1.0 / d)};
+  if (q.p2 && q.r >= 0x1p-100 && q.r <= 0x1p+100)
+    q.as = 2;
+  else if ((double)q.fd == d && d >= 0x1p-100 && d <= 0x1p+100)
+    q.as = 1;
+  return q;
+}
 inline DivF make_divf(float d) { return DivF{d, 1.0f / d, host_is_pow2((double)d) ? 1 : 0}; }
 AW_D double ddiv(double x, const DivD &q) { return q.p2 ? dmul(x, q.r) : __ddiv_rn(x, q.d); }
+AW_D float div_float(float x, const DivD &q) {
+  if (q.as == 2) return fmul(x, q.fr);
+  if (q.as == 1) return fdiv(x, q.fd);
+  return __double2float_rn(ddiv((double)x, q));
+}
 AW_D float fdivq(float x, const DivF &q) { return q.p2 ? fmul(x, q.r) : fdiv(x, q.d); }
 
 // Atlas subjects on grids of their own: a deformation lives on the template
@@ -111,6 +130,37 @@ AW_D int ref_floor_f(float x) {
   int f = __float2int_rz(x);
   if (x < 0.0f && x != __int2float_rn(f)) --f;
   return f;
+}
+
+// The cell of a position and its float corner, as ref_floor_f finds them,
+// without the conversion unit, which the interpolation kernels' 24 float to
+// double conversions a voxel keep half busy: adding 1.5 * 2^23 rounds to the
+// nearest integer in the mantissa's low bits, and a value it rounded up steps
+// back down. For positions within 2^21 of zero; others (huge, infinite, NaN)
+// take ref_floor_f.
+AW_D void floor_near(float x, int &i, float &f) {
+  const float t = fadd(x, 12582912.0f);
+  f = fsub(t, 12582912.0f);
+  i = __float_as_int(t) - 0x4b400000;
+  if (f > x) {
+    f = fsub(f, 1.0f);
+    --i;
+  }
+}
+AW_D void cell_of(float x, float y, float z, int &fx, int &fy, int &fz, float &gx, float &gy,
+                  float &gz) {
+  if (fadd(fadd(fabsf(x), fabsf(y)), fabsf(z)) < 2097152.0f) {
+    floor_near(x, fx, gx);
+    floor_near(y, fy, gy);
+    floor_near(z, fz, gz);
+  } else {
+    fx = ref_floor_f(x);
+    fy = ref_floor_f(y);
+    fz = ref_floor_f(z);
+    gx = __int2float_rn(fx);
+    gy = __int2float_rn(fy);
+    gz = __int2float_rn(fz);
+  }
 }
 
 // ((omt*(omu*(c0*omv + c7*v) + u*(c3*omv + c4*v))) + t*(omu*(c1*omv + c6*v) + u*(c2*omv + c5*v)))
@@ -174,6 +224,80 @@ AW_D float trilerp_scalar(const float *__restrict__ a, const Dims d, double x, d
   return __double2float_rn(lerp_tree(c, t, u, v, omt, omu, omv));
 }
 
+// The eight corners of a cell on a grid: clamped offsets, and which corners
+// lie inside.
+struct CellCorners {
+  int x[2], y[2], z[2];      // offsets along each axis
+  bool ix[2], iy[2], iz[2];
+  AW_D int at(int c) const { return z[kZ(c)] + y[kY(c)] + x[kX(c)]; }
+  AW_D bool in(int c) const { return ix[kX(c)] && iy[kY(c)] && iz[kZ(c)]; }
+  // corner c of the reference's order is (x, y, z) = (kX, kY, kZ)
+  AW_D static constexpr int kX(int c) { return (0x66 >> c) & 1; }
+  AW_D static constexpr int kY(int c) { return (0x3c >> c) & 1; }
+  AW_D static constexpr int kZ(int c) { return (0xf0 >> c) & 1; }
+};
+AW_D CellCorners cell_corners(const Dims &d, int fx, int fy, int fz) {
+  CellCorners k;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    k.x[i] = min(max(fx + i, 0), d.nx - 1);
+    k.y[i] = min(max(fy + i, 0), d.ny - 1) * d.nx;
+    k.z[i] = min(max(fz + i, 0), d.nz - 1) * (d.nx * d.ny);
+    k.ix[i] = (unsigned)(fx + i) < (unsigned)d.nx;
+    k.iy[i] = (unsigned)(fy + i) < (unsigned)d.ny;
+    k.iz[i] = (unsigned)(fz + i) < (unsigned)d.nz;
+  }
+  return k;
+}
+AW_D bool cell_inside(const Dims &d, int fx, int fy, int fz) {
+  return (unsigned)fx < (unsigned)(d.nx - 1) && (unsigned)fy < (unsigned)(d.ny - 1) &&
+         (unsigned)fz < (unsigned)(d.nz - 1);
+}
+// whether any of the warp's threads here has p: kernels whose common case
+// and border case differ choose one for the whole warp, so that a warp with
+// a single border voxel does not run both, one after the other
+AW_D bool warp_any(bool p) { return __any_sync(__activemask(), p); }
+
+// The same at a float position. A cell inside the volume has no negative
+// coordinate, and x - floor(x) of a float x >= 0 is a float: there the
+// fractions are formed in float and widened. A warp with a cell at the
+// border fetches clamped corners and selects.
+template <bool FAST = false>
+AW_D float trilerp_scalar(const float *__restrict__ a, const Dims d, float x, float y, float z,
+                          float bg) {
+  int fx, fy, fz;
+  float gx, gy, gz;
+  cell_of(x, y, z, fx, fy, fz, gx, gy, gz);
+  float c[8];
+  double t, u, v;
+  if (!warp_any(!cell_inside(d, fx, fy, fz))) {
+    const int b = (fz * d.ny + fy) * d.nx + fx;
+    const int sy = d.nx, sz = d.nx * d.ny;
+    c[0] = __ldg(a + b);
+    c[1] = __ldg(a + b + 1);
+    c[2] = __ldg(a + b + sy + 1);
+    c[3] = __ldg(a + b + sy);
+    c[4] = __ldg(a + b + sy + sz);
+    c[5] = __ldg(a + b + sy + sz + 1);
+    c[6] = __ldg(a + b + sz + 1);
+    c[7] = __ldg(a + b + sz);
+    t = (double)fsub(x, gx);
+    u = (double)fsub(y, gy);
+    v = (double)fsub(z, gz);
+  } else {
+    const CellCorners k = cell_corners(d, fx, fy, fz);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) c[i] = __ldg(a + k.at(i));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) c[i] = k.in(i) ? c[i] : bg;
+    t = dsub((double)x, (double)gx);
+    u = dsub((double)y, (double)gy);
+    v = dsub((double)z, (double)gz);
+  }
+  if (FAST) return lerp_tree_f(c, (float)t, (float)u, (float)v);
+  return __double2float_rn(lerp_tree(c, t, u, v, dsub(1.0, t), dsub(1.0, u), dsub(1.0, v)));
+}
+
 AW_D int safe_mod(int r, int m) {
   r %= m;
   return r < 0 ? r + m : r;
@@ -189,56 +313,35 @@ template <bool FAST = false>
 AW_D void trilerp_vector(const float *__restrict__ hx, const float *__restrict__ hy,
                          const float *__restrict__ hz, const Dims d, float x, float y, float z,
                          int bgs, float scale, float &ox, float &oy, float &oz) {
-  int fx = ref_floor_f(x), fy = ref_floor_f(y), fz = ref_floor_f(z);
-  int cx = fx + 1, cy = fy + 1, cz = fz + 1;
-  const float tf = fsub(x, __int2float_rn(fx));
-  const float uf = fsub(y, __int2float_rn(fy));
-  const float vf = fsub(z, __int2float_rn(fz));
+  int fx, fy, fz;
+  float gx, gy, gz;
+  cell_of(x, y, z, fx, fy, fz, gx, gy, gz);
+  const float tf = fsub(x, gx), uf = fsub(y, gy), vf = fsub(z, gz);
   const double t = (double)tf, u = (double)uf, v = (double)vf;
   const double omt = FAST ? 0.0 : dsub(1.0, t), omu = FAST ? 0.0 : dsub(1.0, u),
                omv = FAST ? 0.0 : dsub(1.0, v);
-  bool inside = true;
-  if (bgs == BG_WRAP) {
-    fx = safe_mod(fx, d.nx); fy = safe_mod(fy, d.ny); fz = safe_mod(fz, d.nz);
-    cx = safe_mod(cx, d.nx); cy = safe_mod(cy, d.ny); cz = safe_mod(cz, d.nz);
-  } else if (bgs == BG_CLAMP) {
-    if (fx < 0) { fx = 0; if (cx < 0) cx = 0; }
-    if (cx >= d.nx) { cx = d.nx - 1; if (fx >= d.nx) fx = d.nx - 1; }
-    if (fy < 0) { fy = 0; if (cy < 0) cy = 0; }
-    if (cy >= d.ny) { cy = d.ny - 1; if (fy >= d.ny) fy = d.ny - 1; }
-    if (fz < 0) { fz = 0; if (cz < 0) cz = 0; }
-    if (cz >= d.nz) { cz = d.nz - 1; if (fz >= d.nz) fz = d.nz - 1; }
-  } else {
-    inside = fx >= 0 && cx < d.nx && fy >= 0 && cy < d.ny && fz >= 0 && cz < d.nz;
-  }
-  const int X[8] = {fx, cx, cx, fx, fx, cx, cx, fx};
-  const int Y[8] = {fy, fy, cy, cy, cy, cy, fy, fy};
-  const int Z[8] = {fz, fz, fz, fz, cz, cz, cz, cz};
   float cxv[8], cyv[8], czv[8];
-  if (inside) {
-    // corner offsets from one 32-bit base (grids have < 2^31 voxels); CLAMP
-    // and WRAP corners are not a unit cube, so they index each corner
-    const int sy = d.nx, sz = d.nx * d.ny;
-    int off[8];
-    if (bgs == BG_WRAP || bgs == BG_CLAMP) {
-#pragma unroll
-      for (int c = 0; c < 8; ++c) off[c] = (Z[c] * d.ny + Y[c]) * d.nx + X[c];
+  if (bgs == BG_WRAP || bgs == BG_CLAMP) {
+    int cx = fx + 1, cy = fy + 1, cz = fz + 1;
+    if (bgs == BG_WRAP) {
+      fx = safe_mod(fx, d.nx); fy = safe_mod(fy, d.ny); fz = safe_mod(fz, d.nz);
+      cx = safe_mod(cx, d.nx); cy = safe_mod(cy, d.ny); cz = safe_mod(cz, d.nz);
     } else {
-      const int b = (fz * d.ny + fy) * d.nx + fx;
-      off[0] = b;
-      off[1] = b + 1;
-      off[2] = b + sy + 1;
-      off[3] = b + sy;
-      off[4] = b + sy + sz;
-      off[5] = b + sy + sz + 1;
-      off[6] = b + sz + 1;
-      off[7] = b + sz;
+      if (fx < 0) { fx = 0; if (cx < 0) cx = 0; }
+      if (cx >= d.nx) { cx = d.nx - 1; if (fx >= d.nx) fx = d.nx - 1; }
+      if (fy < 0) { fy = 0; if (cy < 0) cy = 0; }
+      if (cy >= d.ny) { cy = d.ny - 1; if (fy >= d.ny) fy = d.ny - 1; }
+      if (fz < 0) { fz = 0; if (cz < 0) cz = 0; }
+      if (cz >= d.nz) { cz = d.nz - 1; if (fz >= d.nz) fz = d.nz - 1; }
     }
+    const int X[2] = {fx, cx}, Y[2] = {fy, cy}, Z[2] = {fz, cz};
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      cxv[c] = __ldg(hx + off[c]);
-      cyv[c] = __ldg(hy + off[c]);
-      czv[c] = __ldg(hz + off[c]);
+      const int i = (Z[CellCorners::kZ(c)] * d.ny + Y[CellCorners::kY(c)]) * d.nx +
+                    X[CellCorners::kX(c)];
+      cxv[c] = __ldg(hx + i);
+      cyv[c] = __ldg(hy + i);
+      czv[c] = __ldg(hz + i);
     }
     if (scale != 1.0f) {
 #pragma unroll
@@ -248,28 +351,53 @@ AW_D void trilerp_vector(const float *__restrict__ hx, const float *__restrict__
         czv[c] = fmul(czv[c], scale);
       }
     }
-  } else if (bgs == BG_ID) {
-    ox = x; oy = y; oz = z;
-    return;
-  } else if (bgs == BG_ZERO) {
-    ox = 0.f; oy = 0.f; oz = 0.f;
-    return;
   } else {
-    const bool pid = (bgs == BG_PARTIAL_ID);
+    const bool inside = cell_inside(d, fx, fy, fz);
+    if (!inside && (bgs == BG_ID || bgs == BG_ZERO)) {
+      ox = bgs == BG_ID ? x : 0.f;
+      oy = bgs == BG_ID ? y : 0.f;
+      oz = bgs == BG_ID ? z : 0.f;
+      return;
+    }
+    if (!warp_any(!inside)) {
+      const int b = (fz * d.ny + fy) * d.nx + fx;
+      const int sy = d.nx, sz = d.nx * d.ny;
+      const int off[8] = {b, b + 1, b + sy + 1, b + sy, b + sy + sz, b + sy + sz + 1, b + sz + 1,
+                          b + sz};
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const bool in = X[c] >= 0 && X[c] < d.nx && Y[c] >= 0 && Y[c] < d.ny && Z[c] >= 0 && Z[c] < d.nz;
-      if (in) {
-        const long i = d.idx(X[c], Y[c], Z[c]);
+      for (int c = 0; c < 8; ++c) {
+        cxv[c] = __ldg(hx + off[c]);
+        cyv[c] = __ldg(hy + off[c]);
+        czv[c] = __ldg(hz + off[c]);
+      }
+      if (scale != 1.0f) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          cxv[c] = fmul(cxv[c], scale);
+          cyv[c] = fmul(cyv[c], scale);
+          czv[c] = fmul(czv[c], scale);
+        }
+      }
+    } else {
+      // a border cell in the warp: clamped corners, and outside the volume
+      // the corner's own place (PARTIAL_ID) or zero
+      const CellCorners k = cell_corners(d, fx, fy, fz);
+      const bool pid = bgs == BG_PARTIAL_ID;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const int i = k.at(c);
         cxv[c] = fmul(__ldg(hx + i), scale);
         cyv[c] = fmul(__ldg(hy + i), scale);
         czv[c] = fmul(__ldg(hz + i), scale);
-      } else if (pid) {
-        cxv[c] = __int2float_rn(X[c]);
-        cyv[c] = __int2float_rn(Y[c]);
-        czv[c] = __int2float_rn(Z[c]);
-      } else {
-        cxv[c] = 0.f; cyv[c] = 0.f; czv[c] = 0.f;
+      }
+      const float X[2] = {gx, __int2float_rn(fx + 1)}, Y[2] = {gy, __int2float_rn(fy + 1)},
+                  Z[2] = {gz, __int2float_rn(fz + 1)};
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const bool in = k.in(c);
+        cxv[c] = in ? cxv[c] : (pid ? X[CellCorners::kX(c)] : 0.f);
+        cyv[c] = in ? cyv[c] : (pid ? Y[CellCorners::kY(c)] : 0.f);
+        czv[c] = in ? czv[c] : (pid ? Z[CellCorners::kZ(c)] : 0.f);
       }
     }
   }

@@ -78,14 +78,14 @@ struct SrcForce {
   const float *B;
   int mode;
   DivD c2[3], c1[3];  // 2 sp and sp per axis
-  // All six divisors are powers of two whose reciprocals are normal floats:
-  // the difference times the float reciprocal is then the same float as the
-  // double quotient rounded (both are the exact product, rounded once to
-  // nearest), so the gradient needs no double arithmetic.
-  int fexact;
-  float r2[3], r1[3];
+  // how all six divisors divide (DivD::as, the least of theirs), with the
+  // float divisors (1) or reciprocals (2) at hand: one uniform choice and no
+  // lookup of the whole divisor a voxel
+  int as;
+  float f2[3], f1[3];
   AW_D float grad(float diff, int comp, bool interior) const {
-    if (fexact) return fmul(diff, interior ? r2[comp] : r1[comp]);
+    if (as == 2) return fmul(diff, interior ? f2[comp] : f1[comp]);
+    if (as == 1) return fdiv(diff, interior ? f2[comp] : f1[comp]);
     return __double2float_rn(ddiv((double)diff, interior ? c2[comp] : c1[comp]));
   }
   // M from preloaded values (b is read only in mode 2)
@@ -244,15 +244,16 @@ inline SrcForce make_force(const float *G, const float *A, int mode, const Spaci
   f.B = B;
   f.mode = mode;
   const double s[3] = {sp.x, sp.y, sp.z};
-  f.fexact = 1;
+  f.as = 2;
   for (int c = 0; c < 3; ++c) {
     f.c2[c] = make_div(2.0 * s[c]);
     f.c1[c] = make_div(s[c]);
-    f.r2[c] = (float)f.c2[c].r;
-    f.r1[c] = (float)f.c1[c].r;
-    // a power of two whose reciprocal is a float (well inside the normal range)
-    for (const DivD *q : {&f.c2[c], &f.c1[c]})
-      if (!q->p2 || !(q->r >= 0x1p-100 && q->r <= 0x1p+100)) f.fexact = 0;
+    for (const DivD *q : {&f.c2[c], &f.c1[c]}) f.as = q->as < f.as ? q->as : f.as;
+  }
+  for (int c = 0; c < 3; ++c) {
+    // a power of two is a float too, so the least kind serves all six
+    f.f2[c] = f.as == 2 ? f.c2[c].fr : f.c2[c].fd;
+    f.f1[c] = f.as == 2 ? f.c1[c].fr : f.c1[c].fd;
   }
   return f;
 }

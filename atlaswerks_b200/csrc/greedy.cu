@@ -55,9 +55,14 @@ __global__ void __launch_bounds__(kRowThreads)
     const int y1 = min(y0 + kPrepRows, d.ny);
     for (int y = y0; y < y1; ++y) {
       const long i = ((long)z * d.ny + y) * d.nx + x;
-      double px = (double)hx[i], py = (double)hy[i], pz = (double)hz[i];
-      if (AFFINE) atlas_point(am, px, py, pz);
-      const float v = trilerp_scalar<FAST>(I0, AFFINE ? di : d, px, py, pz, 0.0f);
+      float v;
+      if (AFFINE) {
+        double px = (double)hx[i], py = (double)hy[i], pz = (double)hz[i];
+        atlas_point(am, px, py, pz);
+        v = trilerp_scalar<FAST>(I0, di, px, py, pz, 0.0f);
+      } else {
+        v = trilerp_scalar<FAST>(I0, d, hx[i], hy[i], hz[i], 0.0f);
+      }
       idef[i] = v;
       const float r = -fsub(v, I1[i]);
       e += (double)r * (double)r;
@@ -197,10 +202,10 @@ __global__ void __launch_bounds__(kRowThreads)
 // voxel reads lie within one voxel of it: a CTA owns a 32 x TY x TZ tile and
 // the three components of h over the tile plus a one-voxel halo arrive by
 // TMA tensor loads (x from x0 - 4, so the box starts on a 16-byte boundary:
-// 40 x (TY+2) x (TZ+2) floats each). Corners inside the volume and the box
-// are read from shared memory with trilerp_vector's own arithmetic (corner
-// order, double weights, lerp tree); any other voxel (a corner outside the
-// volume, a larger step) takes trilerp_vector from global memory. No inverse
+// 40 x (TY+2) x (TZ+2) floats each). Cells inside the box are read from
+// shared memory with trilerp_vector's own arithmetic (corner order, double
+// weights, lerp tree; a corner outside the volume is its own place); a voxel
+// beyond the box (a larger step) takes trilerp_vector from global memory. No inverse
 // field. The tile shape is chosen per grid by timing (tune_update_tile).
 constexpr int kUTX = 32, kUBX = 40;
 template <int TY, int TZ>
@@ -260,17 +265,14 @@ __global__ void __launch_bounds__(kUTX * TY, 1024 / (kUTX * TY))
     const float px = fadd(__int2float_rn(x), fdivq(fmul(vx4[zz], eps), a.q0));
     const float py = fadd(__int2float_rn(y), fdivq(fmul(vy4[zz], eps), a.q1));
     const float pz = fadd(__int2float_rn(z), fdivq(fmul(vz4[zz], eps), a.q2));
-    const int fx = ref_floor_f(px), fy = ref_floor_f(py), fz = ref_floor_f(pz);
-    const bool fast = staged && fx >= 0 && fx + 1 < d.nx && fy >= 0 && fy + 1 < d.ny &&
-                      fz >= 0 && fz + 1 < d.nz && fx >= bx0 && fx + 1 < bx0 + kUBX &&
-                      fy >= by0 && fy + 1 < by0 + kUBY && fz >= bz0 && fz + 1 < bz0 + kUBZ;
+    int fx, fy, fz;
+    float gx, gy, gz;
+    cell_of(px, py, pz, fx, fy, fz, gx, gy, gz);
+    const int ox = fx - bx0, oy = fy - by0, oz = fz - bz0;  // the cell in the staged box
     float rx, ry, rz;
-    if (fast) {
-      const double tt = (double)fsub(px, __int2float_rn(fx));
-      const double uu = (double)fsub(py, __int2float_rn(fy));
-      const double vv = (double)fsub(pz, __int2float_rn(fz));
-      const double omt = dsub(1.0, tt), omu = dsub(1.0, uu), omv = dsub(1.0, vv);
-      const int b = ((fz - bz0) * kUBY + (fy - by0)) * kUBX + (fx - bx0);
+    if (staged && (unsigned)ox < kUBX - 1 && (unsigned)oy < kUBY - 1 && (unsigned)oz < kUBZ - 1) {
+      const float tf = fsub(px, gx), uf = fsub(py, gy), vf = fsub(pz, gz);
+      const int b = (oz * kUBY + oy) * kUBX + ox;
       constexpr int sy = kUBX, sz = kUBX * kUBY;
       const int off[8] = {b, b + 1, b + sy + 1, b + sy, b + sy + sz, b + sy + sz + 1, b + sz + 1,
                           b + sz};
@@ -281,6 +283,21 @@ __global__ void __launch_bounds__(kUTX * TY, 1024 / (kUTX * TY))
         cy[c] = sh[1][off[c]];
         cz[c] = sh[2][off[c]];
       }
+      if (warp_any(!cell_inside(d, fx, fy, fz))) {
+        // corners outside the volume (zeros in the box) are their own place
+        const float X[2] = {gx, fadd(gx, 1.0f)}, Y[2] = {gy, fadd(gy, 1.0f)},
+                    Z[2] = {gz, fadd(gz, 1.0f)};
+        const CellCorners k = cell_corners(d, fx, fy, fz);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const bool in = k.in(c);
+          cx[c] = in ? cx[c] : X[CellCorners::kX(c)];
+          cy[c] = in ? cy[c] : Y[CellCorners::kY(c)];
+          cz[c] = in ? cz[c] : Z[CellCorners::kZ(c)];
+        }
+      }
+      const double tt = (double)tf, uu = (double)uf, vv = (double)vf;
+      const double omt = dsub(1.0, tt), omu = dsub(1.0, uu), omv = dsub(1.0, vv);
       rx = __double2float_rn(lerp_tree(cx, tt, uu, vv, omt, omu, omv));
       ry = __double2float_rn(lerp_tree(cy, tt, uu, vv, omt, omu, omv));
       rz = __double2float_rn(lerp_tree(cz, tt, uu, vv, omt, omu, omv));

@@ -21,34 +21,37 @@ __global__ void __launch_bounds__(kThreads)
   Voxel vx;
   if (!voxel_of(d, vx)) return;
   const long i = vx.i;
-  out[i] = trilerp_scalar(img, d, (double)hx[i], (double)hy[i], (double)hz[i], bg);
+  out[i] = trilerp_scalar(img, d, hx[i], hy[i], hz[i], bg);
 }
+
+struct AxisDiv {
+  DivD q[3];
+};
 
 // Array3DUtils::computeGradient (Array3DUtils.txx:783-900)
 __global__ void __launch_bounds__(kThreads)
     k_gradient(const float *__restrict__ a, float *__restrict__ gx, float *__restrict__ gy,
-               float *__restrict__ gz, Dims d, Spacing sp, int wrap) {
+               float *__restrict__ gz, Dims d, AxisDiv c2, AxisDiv c1, int wrap) {
   Voxel vx;
   if (!voxel_of(d, vx)) return;
   const long i = vx.i;
   const int pos[3] = {vx.x, vx.y, vx.z};
   const int n[3] = {d.nx, d.ny, d.nz};
   const long stride[3] = {1, d.nx, (long)d.nx * d.ny};
-  const double s[3] = {sp.x, sp.y, sp.z};
   float *g[3] = {gx, gy, gz};
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     float r;
     if (pos[c] > 0 && pos[c] < n[c] - 1) {
-      r = __double2float_rn((double)fsub(a[i + stride[c]], a[i - stride[c]]) / (2.0 * s[c]));
+      r = div_float(fsub(a[i + stride[c]], a[i - stride[c]]), c2.q[c]);
     } else if (wrap) {
       const long ip = pos[c] == n[c] - 1 ? i - (long)(n[c] - 1) * stride[c] : i + stride[c];
       const long im = pos[c] == 0 ? i + (long)(n[c] - 1) * stride[c] : i - stride[c];
-      r = __double2float_rn((double)fsub(a[ip], a[im]) / (2.0 * s[c]));
+      r = div_float(fsub(a[ip], a[im]), c2.q[c]);
     } else if (pos[c] == 0) {
-      r = __double2float_rn((double)fsub(a[i + stride[c]], a[i]) / s[c]);
+      r = div_float(fsub(a[i + stride[c]], a[i]), c1.q[c]);
     } else {
-      r = __double2float_rn((double)fsub(a[i], a[i - stride[c]]) / s[c]);
+      r = div_float(fsub(a[i], a[i - stride[c]]), c1.q[c]);
     }
     g[c][i] = r;
   }
@@ -60,15 +63,16 @@ __global__ void __launch_bounds__(kThreads)
     k_compose_hv(const float *__restrict__ gx, const float *__restrict__ gy, const float *__restrict__ gz,
                  const float *__restrict__ vx, const float *__restrict__ vy, const float *__restrict__ vz,
                  float *__restrict__ ox, float *__restrict__ oy, float *__restrict__ oz, Dims d,
-                 Spacing sp, int dir, int bgs, const float *__restrict__ scale_ptr, float scale_val) {
+                 DivF q0, DivF q1, DivF q2, int dir, int bgs, const float *__restrict__ scale_ptr,
+                 float scale_val) {
   Voxel vox;
   if (!voxel_of(d, vox)) return;
   const long i = vox.i;
   const int x = vox.x, y = vox.y, z = vox.z;
   const float scale = scale_ptr ? *scale_ptr : scale_val;
-  const float dx = fdiv(fmul(vx[i], scale), (float)sp.x);
-  const float dy = fdiv(fmul(vy[i], scale), (float)sp.y);
-  const float dz = fdiv(fmul(vz[i], scale), (float)sp.z);
+  const float dx = fdivq(fmul(vx[i], scale), q0);
+  const float dy = fdivq(fmul(vy[i], scale), q1);
+  const float dz = fdivq(fmul(vz[i], scale), q2);
   float px, py, pz;
   if (dir > 0) {
     px = fadd(__int2float_rn(x), dx); py = fadd(__int2float_rn(y), dy); pz = fadd(__int2float_rn(z), dz);
@@ -88,7 +92,8 @@ __global__ void __launch_bounds__(kThreads)
     k_compose_vh(const float *__restrict__ vx, const float *__restrict__ vy, const float *__restrict__ vz,
                  const float *__restrict__ gx, const float *__restrict__ gy, const float *__restrict__ gz,
                  float *__restrict__ ox, float *__restrict__ oy, float *__restrict__ oz, Dims d,
-                 Spacing sp, int dir, int bgs, const float *__restrict__ scale_ptr, float scale_val) {
+                 DivF q0, DivF q1, DivF q2, int dir, int bgs, const float *__restrict__ scale_ptr,
+                 float scale_val) {
   Voxel vox;
   if (!voxel_of(d, vox)) return;
   const long i = vox.i;
@@ -96,11 +101,9 @@ __global__ void __launch_bounds__(kThreads)
   const float g0 = gx[i], g1 = gy[i], g2 = gz[i];
   float hx, hy, hz;
   trilerp_vector(vx, vy, vz, d, g0, g1, g2, bgs, scale, hx, hy, hz);
-  const float sx = (float)sp.x, sy = (float)sp.y, sz = (float)sp.z;
-  if (dir > 0) {
-    hx = fdiv(hx, sx); hy = fdiv(hy, sy); hz = fdiv(hz, sz);
-  } else {
-    hx = fdiv(hx, -sx); hy = fdiv(hy, -sy); hz = fdiv(hz, -sz);
+  hx = fdivq(hx, q0); hy = fdivq(hy, q1); hz = fdivq(hz, q2);
+  if (dir <= 0) {  // a / -s = -(a / s) exactly in round-to-nearest
+    hx = -hx; hy = -hy; hz = -hz;
   }
   ox[i] = fadd(hx, g0);
   oy[i] = fadd(hy, g1);
@@ -117,7 +120,9 @@ cudaError_t launch_apply(const float *img, const float *hx, const float *hy, con
 
 cudaError_t launch_gradient(const float *a, float *gx, float *gy, float *gz, Dims d, Spacing sp,
                             int wrap, cudaStream_t s) {
-  k_gradient<<<row_grid(d), kThreads, 0, s>>>(a, gx, gy, gz, d, sp, wrap);
+  const AxisDiv c2{{make_div(2.0 * sp.x), make_div(2.0 * sp.y), make_div(2.0 * sp.z)}};
+  const AxisDiv c1{{make_div(sp.x), make_div(sp.y), make_div(sp.z)}};
+  k_gradient<<<row_grid(d), kThreads, 0, s>>>(a, gx, gy, gz, d, c2, c1, wrap);
   return cudaGetLastError();
 }
 
@@ -125,7 +130,9 @@ cudaError_t launch_compose_hv(const float *const g[3], const float *const v[3], 
                               Dims d, Spacing sp, int dir, int bgs, const float *scale_ptr,
                               float scale_val, cudaStream_t s) {
   k_compose_hv<<<row_grid(d), kThreads, 0, s>>>(g[0], g[1], g[2], v[0], v[1], v[2], o[0], o[1],
-                                                    o[2], d, sp, dir, bgs, scale_ptr, scale_val);
+                                                    o[2], d, make_divf((float)sp.x), make_divf((float)sp.y),
+                                                    make_divf((float)sp.z), dir, bgs, scale_ptr,
+                                                    scale_val);
   return cudaGetLastError();
 }
 
@@ -133,7 +140,9 @@ cudaError_t launch_compose_vh(const float *const v[3], const float *const g[3], 
                               Dims d, Spacing sp, int dir, int bgs, const float *scale_ptr,
                               float scale_val, cudaStream_t s) {
   k_compose_vh<<<row_grid(d), kThreads, 0, s>>>(v[0], v[1], v[2], g[0], g[1], g[2], o[0], o[1],
-                                                    o[2], d, sp, dir, bgs, scale_ptr, scale_val);
+                                                    o[2], d, make_divf((float)sp.x), make_divf((float)sp.y),
+                                                    make_divf((float)sp.z), dir, bgs, scale_ptr,
+                                                    scale_val);
   return cudaGetLastError();
 }
 

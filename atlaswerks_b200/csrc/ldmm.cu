@@ -34,6 +34,14 @@ __global__ void __launch_bounds__(kRowThreads)
   hz[v.i] = __int2float_rn(v.z);
 }
 
+// the float spacing's divisions (exact scalings where it is a power of two)
+struct SpaceDiv {
+  DivF x, y, z;
+};
+SpaceDiv space_div(const Spacing &sp) {
+  return SpaceDiv{make_divf((float)sp.x), make_divf((float)sp.y), make_divf((float)sp.z)};
+}
+
 // h_out(x) = h_in(x - v(x)/sp) [PARTIAL_ID]; J(x) = I0(h_out(x))
 // (composeHVInv + apply, LDMMIteratorCPU.cxx:549-554); with PLUS,
 // h_in(x + v(x)/sp) (composeHV, IterateOrig's backward sweep :397-405)
@@ -43,12 +51,11 @@ __global__ void __launch_bounds__(kRowThreads)
                    const float *__restrict__ hz, const float *__restrict__ vx,
                    const float *__restrict__ vy, const float *__restrict__ vz,
                    float *__restrict__ ox, float *__restrict__ oy, float *__restrict__ oz,
-                   const float *__restrict__ I0, float *__restrict__ J, Dims d, Spacing sp) {
+                   const float *__restrict__ I0, float *__restrict__ J, Dims d, SpaceDiv sp) {
   Voxel vox;
   if (!voxel_of(d, vox)) return;
   const long i = vox.i;
-  const float ux = fdiv(vx[i], (float)sp.x), uy = fdiv(vy[i], (float)sp.y),
-              uz = fdiv(vz[i], (float)sp.z);
+  const float ux = fdivq(vx[i], sp.x), uy = fdivq(vy[i], sp.y), uz = fdivq(vz[i], sp.z);
   const float px = PLUS ? fadd(__int2float_rn(vox.x), ux) : fsub(__int2float_rn(vox.x), ux);
   const float py = PLUS ? fadd(__int2float_rn(vox.y), uy) : fsub(__int2float_rn(vox.y), uy);
   const float pz = PLUS ? fadd(__int2float_rn(vox.z), uz) : fsub(__int2float_rn(vox.z), uz);
@@ -57,7 +64,7 @@ __global__ void __launch_bounds__(kRowThreads)
   ox[i] = a;
   oy[i] = b;
   oz[i] = c;
-  if (J) J[i] = trilerp_scalar(I0, d, (double)a, (double)b, (double)c, 0.0f);
+  if (J) J[i] = trilerp_scalar(I0, d, a, b, c, 0.0f);
 }
 
 // float component c of IterateOrig's world-coordinate map x*sp + v
@@ -80,13 +87,10 @@ AW_D float world_grad(const float *__restrict__ vc, int c, int axis, int x, int 
   // the neighbours' own coordinate along c moves only when axis == c
   const int dlo = (axis == c) ? -1 : 0, dhi = (axis == c) ? 1 : 0;
   if (pos > 0 && pos < n - 1)
-    return __double2float_rn(ddiv((double)fsub(world(vc, i + st, cc + dhi, spc),
-                                                world(vc, i - st, cc + dlo, spc)), c2));
+    return div_float(fsub(world(vc, i + st, cc + dhi, spc), world(vc, i - st, cc + dlo, spc)), c2);
   if (pos == 0)
-    return __double2float_rn(ddiv((double)fsub(world(vc, i + st, cc + dhi, spc),
-                                                world(vc, i, cc, spc)), c1));
-  return __double2float_rn(ddiv((double)fsub(world(vc, i, cc, spc),
-                                              world(vc, i - st, cc + dlo, spc)), c1));
+    return div_float(fsub(world(vc, i + st, cc + dhi, spc), world(vc, i, cc, spc)), c1);
+  return div_float(fsub(world(vc, i, cc, spc), world(vc, i - st, cc + dlo, spc)), c1);
 }
 
 // JacDet_t = (t < T-1 ? JacDet_{t+1}(x + v_t/sp) : 1) * |D(x*sp + v_t)|
@@ -95,12 +99,12 @@ AW_D float world_grad(const float *__restrict__ vc, int c, int axis, int x, int 
 __global__ void __launch_bounds__(kRowThreads)
     k_jacdet(const float *__restrict__ vx, const float *__restrict__ vy,
              const float *__restrict__ vz, const float *__restrict__ next,
-             float *__restrict__ out, Dims d, Spacing sp, DivD a2, DivD b2, DivD e2, DivD a1,
+             float *__restrict__ out, Dims d, SpaceDiv sp, DivD a2, DivD b2, DivD e2, DivD a1,
              DivD b1, DivD e1) {
   Voxel vox;
   if (!voxel_of(d, vox)) return;
   const int x = vox.x, y = vox.y, z = vox.z;
-  const float s[3] = {(float)sp.x, (float)sp.y, (float)sp.z};
+  const float s[3] = {sp.x.d, sp.y.d, sp.z.d};
   const DivD c2[3] = {a2, b2, e2}, c1[3] = {a1, b1, e1};
   const float *vc[3] = {vx, vy, vz};
   float g[3][3];  // g[c][axis]
@@ -115,10 +119,10 @@ __global__ void __launch_bounds__(kRowThreads)
   const long i = vox.i;
   if (next) {
     // applyU: coord = v/sp + (x,y,z), default scalar background 0
-    const float px = fadd(fdiv(vx[i], s[0]), __int2float_rn(x));
-    const float py = fadd(fdiv(vy[i], s[1]), __int2float_rn(y));
-    const float pz = fadd(fdiv(vz[i], s[2]), __int2float_rn(z));
-    out[i] = fmul(trilerp_scalar(next, d, (double)px, (double)py, (double)pz, 0.0f), jac);
+    const float px = fadd(fdivq(vx[i], sp.x), __int2float_rn(x));
+    const float py = fadd(fdivq(vy[i], sp.y), __int2float_rn(y));
+    const float pz = fadd(fdivq(vz[i], sp.z), __int2float_rn(z));
+    out[i] = fmul(trilerp_scalar(next, d, px, py, pz, 0.0f), jac);
   } else {
     out[i] = jac;
   }
@@ -228,7 +232,7 @@ AW_D GradTaps grad_taps(int c, const Voxel &v, const Dims &d) {
   return GradTaps{pos > 0 ? -st : 0, pos < n - 1 ? st : 0, pos > 0 && pos < n - 1};
 }
 AW_D float grad_of(float diff, int c, const GradTaps &t, const GradDiv &g) {
-  return __double2float_rn(ddiv((double)diff, t.in ? g.c2[c] : g.c1[c]));
+  return div_float(diff, t.in ? g.c2[c] : g.c1[c]);
 }
 // component c of computeGradient(a) at voxel v
 AW_D float ref_grad(const float *__restrict__ a, int c, const Voxel &v, const Dims &d,
@@ -288,8 +292,7 @@ __global__ void __launch_bounds__(kRowThreads)
               Dims d) {
   Voxel v;
   if (!voxel_of(d, v)) return;
-  const float r = trilerp_scalar(src, d, (double)__ldg(hx + v.i), (double)__ldg(hy + v.i),
-                                 (double)__ldg(hz + v.i), 0.0f);
+  const float r = trilerp_scalar(src, d, __ldg(hx + v.i), __ldg(hy + v.i), __ldg(hz + v.i), 0.0f);
   out[v.i] = SUB ? fsub(out[v.i], r) : r;
 }
 
@@ -480,7 +483,7 @@ cudaError_t ldmm_forward(LdmmCtx *c, const float *I0, const float *I1, const flo
     k_forward_step<false><<<row_grid(d), kRowThreads, 0, s>>>(
         comp(H[cur], 0), comp(H[cur], 1), comp(H[cur], 2), vcomp(vi, 0), vcomp(vi, 1),
         vcomp(vi, 2), comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I0,
-        c->J0 + (long)i * n, d, c->sp);
+        c->J0 + (long)i * n, d, space_div(c->sp));
     AW_TRY(cudaGetLastError());
     cur = 1 - cur;
   }
@@ -629,13 +632,13 @@ cudaError_t ldmm_i1_at_0(LdmmCtx *c, const float *I1, const float *v, float *img
     k_forward_step<true><<<row_grid(d), kRowThreads, 0, s>>>(
         comp(H[cur], 0), comp(H[cur], 1), comp(H[cur], 2), vcomp(vt, 0), vcomp(vt, 1),
         vcomp(vt, 2), comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I1,
-        t == 0 ? img : nullptr, d, c->sp);
+        t == 0 ? img : nullptr, d, space_div(c->sp));
     AW_TRY(cudaGetLastError());
     cur = 1 - cur;
     if (jd) {
       k_jacdet<<<row_grid(d), kRowThreads, 0, s>>>(vcomp(vt, 0), vcomp(vt, 1), vcomp(vt, 2),
                                                    t == T - 1 ? nullptr : jbuf(t + 1), jbuf(t),
-                                                   d, c->sp, a2, b2, e2, a1, b1, e1);
+                                                   d, space_div(c->sp), a2, b2, e2, a1, b1, e1);
       AW_TRY(cudaGetLastError());
     }
   }
@@ -869,7 +872,7 @@ static cudaError_t shoot_geodesic(LdmmCtx *c, const float *I0, const float *alph
   auto advance_phiT0 = [&]() -> cudaError_t {  // phiT0 = composeHVInv(phiT0, v), I = I0(phiT0)
     k_forward_step<false><<<row_grid(d), kRowThreads, 0, s>>>(
         comp(B[cb], 0), comp(B[cb], 1), comp(B[cb], 2), comp(v, 0), comp(v, 1), comp(v, 2),
-        comp(B[1 - cb], 0), comp(B[1 - cb], 1), comp(B[1 - cb], 2), I0, I, d, c->sp);
+        comp(B[1 - cb], 0), comp(B[1 - cb], 1), comp(B[1 - cb], 2), I0, I, d, space_div(c->sp));
     cb = 1 - cb;
     return cudaGetLastError();
   };
@@ -1175,7 +1178,7 @@ cudaError_t ldmm_adshoot_iterate(LdmmCtx *c, const float *I0, const float *I1, f
     AW_TRY(splat_gather(c->adSort[t], alpha0, oo[0], oo[1], oo[2], A(t), 0.0f, s));
     k_forward_step<false><<<grid, kRowThreads, 0, s>>>(
         comp(P1(t - 1), 0), comp(P1(t - 1), 1), comp(P1(t - 1), 2), vv[0], vv[1], vv[2],
-        comp(P1(t), 0), comp(P1(t), 1), comp(P1(t), 2), I0, I(t), d, c->sp);
+        comp(P1(t), 0), comp(P1(t), 1), comp(P1(t), 2), I0, I(t), d, space_div(c->sp));
     return cudaGetLastError();
   };
 
@@ -1287,12 +1290,12 @@ cudaError_t ldmm_iterate_orig(LdmmCtx *c, const float *I0, const float *I1, floa
     k_forward_step<true><<<row_grid(d), kRowThreads, 0, s>>>(
         comp(H[cur], 0), comp(H[cur], 1), comp(H[cur], 2), comp(vt, 0), comp(vt, 1), comp(vt, 2),
         comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I1, c->JT + (long)t * n,
-        d, c->sp);
+        d, space_div(c->sp));
     AW_TRY(cudaGetLastError());
     cur = 1 - cur;
     k_jacdet<<<row_grid(d), kRowThreads, 0, s>>>(comp(vt, 0), comp(vt, 1), comp(vt, 2),
                                                  t == T - 1 ? nullptr : c->JD + (long)(t + 1) * n,
-                                                 c->JD + (long)t * n, d, c->sp, a2, b2, e2, a1, b1,
+                                                 c->JD + (long)t * n, d, space_div(c->sp), a2, b2, e2, a1, b1,
                                                  e1);
     AW_TRY(cudaGetLastError());
   }
@@ -1321,7 +1324,7 @@ cudaError_t ldmm_iterate_orig(LdmmCtx *c, const float *I0, const float *I1, floa
     }
     k_forward_step<false><<<row_grid(d), kRowThreads, 0, s>>>(
         comp(H[cur], 0), comp(H[cur], 1), comp(H[cur], 2), comp(vt, 0), comp(vt, 1), comp(vt, 2),
-        comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I0, Sb, d, c->sp);
+        comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I0, Sb, d, space_div(c->sp));
     AW_TRY(cudaGetLastError());
     cur = 1 - cur;
     // the image energy is recorded (and the count advanced) after the sweep
