@@ -48,6 +48,17 @@ AW_D bool voxel_of(const Dims &d, Voxel &v) {
   return v.x < d.nx;
 }
 
+// n / d for 0 <= n < 2^31 by multiply and shift (round-up method)
+struct IdxDiv {
+  uint32_t d, mul, l;
+  AW_D int div(int n) const { return (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> l); }
+};
+inline IdxDiv make_idxdiv(uint32_t d) {
+  uint32_t l = 0;
+  while ((1ull << l) < d) ++l;
+  return IdxDiv{d, (uint32_t)(((1ull << 32) * ((1ull << l) - d)) / d + 1), l};
+}
+
 // ---- exact-rounding arithmetic -------------------------------------------
 AW_D double dmul(double a, double b) { return __dmul_rn(a, b); }
 AW_D double dadd(double a, double b) { return __dadd_rn(a, b); }

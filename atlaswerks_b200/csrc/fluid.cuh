@@ -5,9 +5,9 @@
 //               greedy/LDMM body force computed on the fly) -> real-to-complex
 //               FFT along x (two real rows packed per complex line) -> FFT
 //               along y -> half spectrum to HBM.
-//   z-solve     one CTA per tile of K (ky,kx) columns, all three components:
-//               FFT along z -> per-wavenumber 3x3 Cholesky solve (or multiply)
-//               with 1/N scaling -> inverse FFT along z -> back to HBM.
+//   z-solve     one CTA per tile of (ky,kx) columns, all three components:
+//               FFT along z -> per-wavenumber 3x3 solve (or multiply) with
+//               1/N scaling -> inverse FFT along z -> back to HBM.
 //   xy-inverse  one CTA per (z-slab, component): inverse FFT along y ->
 //               complex-to-real along x -> consumer epilogue (store, or the
 //               LDMM velocity update).
@@ -20,6 +20,7 @@
 
 #include "aw_common.cuh"
 #include "fft_smem.cuh"
+#include "fluid_any.cuh"
 
 namespace aw {
 
@@ -28,16 +29,18 @@ struct FluidPlan {
   Spacing sp;
   float alpha, beta, gamma;
   int nxh;
-  FFTAxis ax, ay, az;
-  float2 *tw;      // device twiddle tables (x | y | z)
-  float *lut;      // device LUT: cos x | sin x | cos y | sin y | cos z | sin z
-  float2 *spec;    // device half spectrum [3][nz][ny][nxh]
-  int pairs_per_batch, cols_per_batch, zcols_per_cta;
-  size_t smem_xy, smem_z;
-  // slabs whose half spectrum does not fit one CTA's shared memory: the xy
-  // transforms run as an x pass and a y pass through the spectrum in HBM
+  FFTAxis ax, ay, az;        // register path: the axes' twiddle tables
+  float2 *tw;                // device twiddle tables (x | y | z)
+  float *lut;                // register path's LUT: cos x | sin x | cos y | sin y | cos z | sin z
+  float2 *spec;              // device half spectrum
+  // any-size path (fluid_any.cu): its plan (host) and its tables (device).
+  // Slabs that do not fit one CTA's shared memory run an x and a y pass
+  // through the spectrum in HBM (split), on pairs_per_batch row pairs and
+  // cols_per_batch columns per CTA; the z pass takes zcols_per_cta columns.
+  AnyPlan *any;
+  uint32_t *any_tables;
   int split;
-  size_t smem_x, smem_y;
+  int pairs_per_batch, cols_per_batch, zcols_per_cta;
   int device;
   // register-FFT path (fluid_fast.cu): power-of-two axes
   int fast;
@@ -50,10 +53,22 @@ struct FluidPlan {
 
 // --- producers for the forward pass ----------------------------------------
 // plain vector field input
+// kPairs: row pairs whose loads the any-size path issues together
 struct SrcField {
+  static constexpr int kPairs = 4;
   const float *c[3];
-  AW_D float value(int comp, int x, int y, int z, const Dims &d) const {
-    return __ldg(c[comp] + d.idx(x, y, z));
+  // slab z of component comp: the rows y and y + H at x, zero past the last row
+  struct Slab {
+    const float *f;
+    int nx, ny, H;
+    AW_D float2 pair(int x, int y) const {
+      const int o = y * nx + x, y1 = y + H;
+      const float a = __ldg(f + o), b = __ldg(f + (y1 < ny ? o + H * nx : o));
+      return make_float2(a, y1 < ny ? b : 0.f);
+    }
+  };
+  AW_D Slab at_slab(int comp, int z, int H, const Dims &d) const {
+    return Slab{(comp == 0 ? c[0] : comp == 1 ? c[1] : c[2]) + d.idx(0, 0, z), d.nx, d.ny, H};
   }
   // rows y0 and y0+1 of slab z at x = t + TX*j, j < E, as (row y0, row y0+1)
   template <int E, int TX>
@@ -73,6 +88,7 @@ struct SrcField {
 // central differences / (2 sp), one-sided at the borders, the float
 // difference divided in double.
 struct SrcForce {
+  static constexpr int kPairs = 2;
   const float *G;
   const float *A;
   const float *B;
@@ -108,6 +124,51 @@ struct SrcForce {
     const float b = mode == 2 ? __ldg(B + i) : 0.f;
     const float g = grad(fsub(gh, gl), comp, pos > 0 && pos < n - 1);
     return fmul(g, mismatch_v(g0, a, b));
+  }
+  // Slab z of component comp: the rows y and y + H at x, as value() forms
+  // them, from offsets within the slab; zero past the last row. Every load
+  // of the pair is issued before the arithmetic.
+  struct Slab {
+    const SrcForce *s;
+    const float *g, *a, *b;  // the slab's first voxel
+    int comp, nx, ny, H;
+    int lo, hi;              // z: the neighbouring slabs' offsets
+    bool in;                 // z: central difference
+    AW_D float2 pair(int x, int y) const {
+      const bool two = y + H < ny;
+      const int y1 = two ? y + H : y, o0 = y * nx + x, o1 = y1 * nx + x;
+      int l0 = lo, h0 = hi, l1 = lo, h1 = hi;
+      bool in0 = in, in1 = in;
+      if (comp == 0) {
+        l0 = l1 = x > 0 ? -1 : 0;
+        h0 = h1 = x < nx - 1 ? 1 : 0;
+        in0 = in1 = x > 0 && x < nx - 1;
+      } else if (comp == 1) {
+        l0 = y > 0 ? -nx : 0;
+        h0 = y < ny - 1 ? nx : 0;
+        in0 = y > 0 && y < ny - 1;
+        l1 = y1 > 0 ? -nx : 0;
+        h1 = y1 < ny - 1 ? nx : 0;
+        in1 = y1 > 0 && y1 < ny - 1;
+      }
+      const float g0 = __ldg(g + o0), gh0 = __ldg(g + o0 + h0), gl0 = __ldg(g + o0 + l0);
+      const float g1 = __ldg(g + o1), gh1 = __ldg(g + o1 + h1), gl1 = __ldg(g + o1 + l1);
+      const float a0 = __ldg(a + o0), a1 = __ldg(a + o1);
+      float b0 = 0.f, b1 = 0.f;
+      if (s->mode == 2) {
+        b0 = __ldg(b + o0);
+        b1 = __ldg(b + o1);
+      }
+      const float v0 = fmul(s->grad(fsub(gh0, gl0), comp, in0), s->mismatch_v(g0, a0, b0));
+      const float v1 = fmul(s->grad(fsub(gh1, gl1), comp, in1), s->mismatch_v(g1, a1, b1));
+      return make_float2(v0, two ? v1 : 0.f);
+    }
+  };
+  AW_D Slab at_slab(int comp, int z, int H, const Dims &d) const {
+    const long o = d.idx(0, 0, z);
+    const int sl = d.nx * d.ny;
+    return Slab{this, G + o,  A + o, B + o, comp, d.nx, d.ny, H, z > 0 ? -sl : 0, z < d.nz - 1 ? sl : 0,
+                z > 0 && z < d.nz - 1};
   }
   // Rows y0 and y0+1 of slab z at x = t + TX*j, j < E, as (row y0, row
   // y0+1): the same values as value(), from row pointers formed once and one
@@ -304,6 +365,16 @@ struct DstAxpbyBound {
     for (int j = 0; j < N; ++j) old[j] = c[i[j]];
 #pragma unroll
     for (int j = 0; j < N; ++j) c[i[j]] = fadd(fmul(vfac, old[j]), fmul(ufac, u[j]));
+  }
+  // the same, without the elements whose index is negative
+  template <int N>
+  AW_D void store_some(const long (&i)[N], const float (&u)[N]) const {
+    float old[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) old[j] = i[j] >= 0 ? c[i[j]] : 0.f;
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (i[j] >= 0) c[i[j]] = fadd(fmul(vfac, old[j]), fmul(ufac, u[j]));
   }
 };
 struct DstAxpby {
