@@ -156,6 +156,7 @@ struct UpdateArgs {
   DivF q0, q1, q2;
 };
 
+template <bool FAST>
 __global__ void __launch_bounds__(kRowThreads)
     k_update(UpdateArgs a, Dims d, const float *__restrict__ step_ptr) {
   Voxel vox;
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(kRowThreads)
   const float py = fadd(__int2float_rn(y), fdivq(fmul(a.vy[i], eps), a.q1));
   const float pz = fadd(__int2float_rn(z), fdivq(fmul(a.vz[i], eps), a.q2));
   float rx, ry, rz;
-  trilerp_vector(a.hx, a.hy, a.hz, d, px, py, pz, BG_PARTIAL_ID, 1.0f, rx, ry, rz);
+  trilerp_vector<FAST>(a.hx, a.hy, a.hz, d, px, py, pz, BG_PARTIAL_ID, 1.0f, rx, ry, rz);
   a.ox[i] = rx;
   a.oy[i] = ry;
   a.oz[i] = rz;
@@ -220,7 +221,7 @@ struct HMaps {
   CUtensorMap m[3];
 };
 
-template <int TY, int TZ>
+template <int TY, int TZ, bool FAST>
 __global__ void __launch_bounds__(kUTX * TY, 1024 / (kUTX * TY))
     k_update_tiled(const __grid_constant__ HMaps maps, UpdateArgs a, Dims d,
                    const float *__restrict__ step_ptr, int *status) {
@@ -296,13 +297,19 @@ __global__ void __launch_bounds__(kUTX * TY, 1024 / (kUTX * TY))
           cz[c] = in ? cz[c] : Z[CellCorners::kZ(c)];
         }
       }
-      const double tt = (double)tf, uu = (double)uf, vv = (double)vf;
-      const double omt = dsub(1.0, tt), omu = dsub(1.0, uu), omv = dsub(1.0, vv);
-      rx = __double2float_rn(lerp_tree(cx, tt, uu, vv, omt, omu, omv));
-      ry = __double2float_rn(lerp_tree(cy, tt, uu, vv, omt, omu, omv));
-      rz = __double2float_rn(lerp_tree(cz, tt, uu, vv, omt, omu, omv));
+      if constexpr (FAST) {
+        rx = lerp_tree_f(cx, tf, uf, vf);
+        ry = lerp_tree_f(cy, tf, uf, vf);
+        rz = lerp_tree_f(cz, tf, uf, vf);
+      } else {
+        const double tt = (double)tf, uu = (double)uf, vv = (double)vf;
+        const double omt = dsub(1.0, tt), omu = dsub(1.0, uu), omv = dsub(1.0, vv);
+        rx = __double2float_rn(lerp_tree(cx, tt, uu, vv, omt, omu, omv));
+        ry = __double2float_rn(lerp_tree(cy, tt, uu, vv, omt, omu, omv));
+        rz = __double2float_rn(lerp_tree(cz, tt, uu, vv, omt, omu, omv));
+      }
     } else {
-      trilerp_vector(a.hx, a.hy, a.hz, d, px, py, pz, BG_PARTIAL_ID, 1.0f, rx, ry, rz);
+      trilerp_vector<FAST>(a.hx, a.hy, a.hz, d, px, py, pz, BG_PARTIAL_ID, 1.0f, rx, ry, rz);
     }
     a.ox[i] = rx;
     a.oy[i] = ry;
@@ -351,26 +358,29 @@ bool h_map(GreedyCtx *g, const float *p, int tile, CUtensorMap *out) {
 
 template <int TY, int TZ>
 void launch_tiled(const HMaps &maps, const UpdateArgs &a, const Dims &d, const float *step,
-                  int *status, cudaStream_t s) {
+                  int *status, bool fast, cudaStream_t s) {
   const unsigned tiles = (unsigned)(((d.nx + kUTX - 1) / kUTX) * ((d.ny + TY - 1) / TY) *
                                     ((d.nz + TZ - 1) / TZ));
-  k_update_tiled<TY, TZ><<<tiles, kUTX * TY, 0, s>>>(maps, a, d, step, status);
+  if (fast)
+    k_update_tiled<TY, TZ, true><<<tiles, kUTX * TY, 0, s>>>(maps, a, d, step, status);
+  else
+    k_update_tiled<TY, TZ, false><<<tiles, kUTX * TY, 0, s>>>(maps, a, d, step, status);
 }
 
 // the staged update with tile shape `tile`; false when h cannot be staged
 // (grid or alignment), so the caller takes the global-gather kernel
 bool launch_update_tiled(GreedyCtx *g, int tile, const UpdateArgs &a, const float *const h[3],
-                         cudaStream_t s) {
+                         bool fast, cudaStream_t s) {
   HMaps maps;
   for (int c = 0; c < 3; ++c)
     if (!h_map(g, h[c], tile, &maps.m[c])) return false;
   const Dims d = g->d;
   int *st = g->plan.status;
   switch (tile) {
-    case 0: launch_tiled<8, 4>(maps, a, d, g->st.step, st, s); break;
-    case 1: launch_tiled<4, 8>(maps, a, d, g->st.step, st, s); break;
-    case 2: launch_tiled<8, 8>(maps, a, d, g->st.step, st, s); break;
-    default: launch_tiled<16, 2>(maps, a, d, g->st.step, st, s); break;
+    case 0: launch_tiled<8, 4>(maps, a, d, g->st.step, st, fast, s); break;
+    case 1: launch_tiled<4, 8>(maps, a, d, g->st.step, st, fast, s); break;
+    case 2: launch_tiled<8, 8>(maps, a, d, g->st.step, st, fast, s); break;
+    default: launch_tiled<16, 2>(maps, a, d, g->st.step, st, fast, s); break;
   }
   return true;
 }
@@ -426,10 +436,10 @@ void tune_update_tile(GreedyCtx *g) {
   float *saved_step = g->st.step;
   g->st.step = step;
   for (int tile = 0; tile < kNumTiles; ++tile) {
-    if (!launch_update_tiled(g, tile, a, hc, 0)) break;
+    if (!launch_update_tiled(g, tile, a, hc, false, 0)) break;
     any = true;
     cudaEventRecord(e0, 0);
-    for (int r = 0; r < 3; ++r) launch_update_tiled(g, tile, a, hc, 0);
+    for (int r = 0; r < 3; ++r) launch_update_tiled(g, tile, a, hc, false, 0);
     cudaEventRecord(e1, 0);
     float ms = 0.f;
     if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess)
@@ -450,6 +460,38 @@ void tune_update_tile(GreedyCtx *g) {
   g->utile = pick;
   std::lock_guard<std::mutex> lock(g_tile_mu);
   g_tile[key] = pick;
+}
+
+// Up to here the inverse transform and the update run as one kernel (v never
+// leaves the chip, one launch less); beyond, the update on its own, with h
+// staged by TMA and its own registers and occupancy, is faster: 32^3 6.1
+// against 6.5 us plus a launch, 64^3 12.7 against 11.8, 128^3 51.7 against
+// 47.2, 128 x 128 x 256 (256 wide: one slab per SM) 184 against 94.
+constexpr long kFuseVoxels = 64L * 64 * 63;
+
+// the update on its own: h staged in shared memory where it can be, else
+// gathered from global memory. fast: the float-tree interpolation, which
+// SetFastInterpolation asks for in the iterations that the fused kernel
+// covers (register-path grids, no inverse field, no step update).
+cudaError_t update_stage(GreedyCtx *g, const float *const h[3], float *const h_out[3],
+                         const float *const hinv[3], float *const hinv_out[3], bool fast,
+                         cudaStream_t s) {
+  const Dims d = g->d;
+  const long n = d.n();
+  float *v[3] = {g->vbuf, g->vbuf + n, g->vbuf + 2 * n};
+  const bool inv = hinv && hinv[0] && hinv_out && hinv_out[0];
+  const UpdateArgs a{h[0], h[1], h[2], v[0], v[1], v[2], h_out[0], h_out[1], h_out[2],
+                     inv ? hinv[0] : nullptr, inv ? hinv[1] : nullptr, inv ? hinv[2] : nullptr,
+                     inv ? hinv_out[0] : nullptr, inv ? hinv_out[1] : nullptr,
+                     inv ? hinv_out[2] : nullptr, make_divf((float)g->sp.x),
+                     make_divf((float)g->sp.y), make_divf((float)g->sp.z)};
+  if (inv || g->no_staged_update || !launch_update_tiled(g, g->utile, a, h, fast, s)) {
+    if (fast)
+      k_update<true><<<row_grid(d), kRowThreads, 0, s>>>(a, d, g->st.step);
+    else
+      k_update<false><<<row_grid(d), kRowThreads, 0, s>>>(a, d, g->st.step);
+  }
+  return cudaGetLastError();
 }
 
 #define AW_TRY(x)                         \
@@ -556,25 +598,15 @@ cudaError_t greedy_stage(GreedyCtx *g, int stage, const float *I0, const float *
       k_set_step<<<1, 1, 0, s>>>(g->maxbits, g->max_pert, g->st.step);
       return cudaGetLastError();
     }
-    case kStageUpdate: {
-      const bool inv = hinv && hinv[0] && hinv_out && hinv_out[0];
-      const UpdateArgs a{h[0], h[1], h[2], v[0], v[1], v[2], h_out[0], h_out[1], h_out[2],
-                         inv ? hinv[0] : nullptr, inv ? hinv[1] : nullptr,
-                         inv ? hinv[2] : nullptr, inv ? hinv_out[0] : nullptr,
-                         inv ? hinv_out[1] : nullptr, inv ? hinv_out[2] : nullptr,
-                         make_divf((float)g->sp.x), make_divf((float)g->sp.y),
-                         make_divf((float)g->sp.z)};
-      if (inv || g->no_staged_update || !launch_update_tiled(g, g->utile, a, h, s))
-        k_update<<<row_grid(d), kRowThreads, 0, s>>>(a, d, g->st.step);
-      return cudaGetLastError();
-    }
+    case kStageUpdate:
+      return update_stage(g, h, h_out, hinv, hinv_out, false, s);
     case kStageInvCompose: {
-      // grids the fused kernel does not take run the two stages it replaces
-      if (!g->plan.fast) {
+      // grids the fused kernel does not take, or takes more slowly, run the
+      // two stages it replaces
+      if (!g->plan.fast || d.n() > kFuseVoxels) {
         AW_TRY(greedy_stage(g, kStageXYInverse, I0, I1, h, h_out, hinv, hinv_out, auto_reduce,
                             solve_inverse, s));
-        return greedy_stage(g, kStageUpdate, I0, I1, h, h_out, nullptr, nullptr, auto_reduce,
-                            solve_inverse, s);
+        return update_stage(g, h, h_out, nullptr, nullptr, g->plan.fast && g->fast_interp, s);
       }
       const ComposeArgs a{h[0], h[1], h[2], h_out[0], h_out[1], h_out[2], g->st.step,
                           make_divf((float)g->sp.x), make_divf((float)g->sp.y),
