@@ -1,4 +1,5 @@
 // splat.cu — deterministic counting-sort splat (see splat.cuh).
+#include <algorithm>
 #include <climits>
 
 #include "splat.cuh"
@@ -21,17 +22,20 @@ AW_D long bucket_of(const Dims &d, float px, float py, float pz) {
   if (!(px > -1.0f && px < (float)d.nx && py > -1.0f && py < (float)d.ny && pz > -1.0f &&
         pz < (float)d.nz))
     return -1;
-  const int fx = ref_floor_f(px), fy = ref_floor_f(py), fz = ref_floor_f(pz);
+  int fx, fy, fz;
+  float gx, gy, gz;
+  cell_of(px, py, pz, fx, fy, fz, gx, gy, gz);
   return ((long)(fz + 1) * (d.ny + 1) + (fy + 1)) * (d.nx + 1) + (fx + 1);
 }
 
+// bucket sizes, and every source's place in its bucket (in arrival order)
 __global__ void __launch_bounds__(kRowThreads)
     k_count(const float *__restrict__ hx, const float *__restrict__ hy, const float *__restrict__ hz,
-            Dims d, int *__restrict__ counts) {
+            Dims d, int *__restrict__ counts, int *__restrict__ place) {
   Voxel v;
   if (!voxel_of(d, v)) return;
   const long b = bucket_of(d, hx[v.i], hy[v.i], hz[v.i]);
-  if (b >= 0) atomicAdd(counts + b, 1);
+  if (b >= 0) place[v.i] = atomicAdd(counts + b, 1);
 }
 
 // block-local exclusive scan of kScanBlock ints held 4 per thread
@@ -135,49 +139,40 @@ __global__ void __launch_bounds__(kScanThreads)
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) x[n] = off + total;
 }
 
-__global__ void __launch_bounds__(kRowThreads)
-    k_scatter(const float *__restrict__ hx, const float *__restrict__ hy,
-              const float *__restrict__ hz, Dims d, const int *__restrict__ offsets,
-              int *__restrict__ cursor, int *__restrict__ order) {
-  Voxel v;
-  if (!voxel_of(d, v)) return;
-  const long b = bucket_of(d, hx[v.i], hy[v.i], hz[v.i]);
-  if (b < 0) return;
-  const int pos = offsets[b] + atomicAdd(cursor + b, 1);
-  order[pos] = (int)v.i;
+// weight of corner (cx, cy, cz) of a source with fractions r, rounded to
+// float as forwardApply writes it (HField3DUtils.txx:1116-1123): the product
+// runs left to right, in double once a (1.0 - r) factor has entered it and
+// in float before, so w110 = (rx*ry in float) * (1.0 - rz) and w111 =
+// rx*ry*rz in float.
+struct Fractions {
+  float rx, ry, rz;
+};
+AW_D Fractions fractions_of(float px, float py, float pz) {
+  int fx, fy, fz;
+  float gx, gy, gz;
+  cell_of(px, py, pz, fx, fy, fz, gx, gy, gz);
+  return Fractions{fsub(px, gx), fsub(py, gy), fsub(pz, gz)};
 }
-
-// weight of corner (cx, cy, cz) of a source at p, rounded to float as
-// forwardApply writes it (HField3DUtils.txx:1116-1123): the product runs left
-// to right, in double once a (1.0 - r) factor has entered it and in float
-// before, so w110 = (rx*ry in float) * (1.0 - rz) and w111 = rx*ry*rz in float.
-AW_D float corner_weight(float px, float py, float pz, int cx, int cy, int cz) {
-  const int fx = ref_floor_f(px), fy = ref_floor_f(py), fz = ref_floor_f(pz);
-  const float rx = fsub(px, __int2float_rn(fx)), ry = fsub(py, __int2float_rn(fy)),
-              rz = fsub(pz, __int2float_rn(fz));
+AW_D float corner_weight(const Fractions &f, int cx, int cy, int cz) {
   if (cx && cy) {
-    const float rxy = fmul(rx, ry);
-    return cz ? fmul(rxy, rz) : __double2float_rn(dmul((double)rxy, dsub(1.0, (double)rz)));
+    const float rxy = fmul(f.rx, f.ry);
+    return cz ? fmul(rxy, f.rz) : __double2float_rn(dmul((double)rxy, dsub(1.0, (double)f.rz)));
   }
-  const double ax = cx ? (double)rx : dsub(1.0, (double)rx);
-  const double ay = cy ? (double)ry : dsub(1.0, (double)ry);
-  const double az = cz ? (double)rz : dsub(1.0, (double)rz);
+  const double ax = cx ? (double)f.rx : dsub(1.0, (double)f.rx);
+  const double ay = cy ? (double)f.ry : dsub(1.0, (double)f.ry);
+  const double az = cz ? (double)f.rz : dsub(1.0, (double)f.rz);
   return __double2float_rn(dmul(dmul(ax, ay), az));
 }
 
-// the eight corner weights (index dx + 2 dy + 4 dz) of the source at sorted
-// position i
-AW_D void store_weights(const int *__restrict__ order, int i, const float *__restrict__ hx,
-                        const float *__restrict__ hy, const float *__restrict__ hz,
-                        float *__restrict__ wts) {
-  const int m = order[i];
-  const float px = __ldg(hx + m), py = __ldg(hy + m), pz = __ldg(hz + m);
-  float w[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) w[k] = corner_weight(px, py, pz, k & 1, (k >> 1) & 1, (k >> 2) & 1);
-  float4 *o = reinterpret_cast<float4 *>(wts + (long)i * 8);
-  o[0] = make_float4(w[0], w[1], w[2], w[3]);
-  o[1] = make_float4(w[4], w[5], w[6], w[7]);
+// sources to their buckets, in arrival order
+__global__ void __launch_bounds__(kRowThreads)
+    k_scatter(const float *__restrict__ hx, const float *__restrict__ hy,
+              const float *__restrict__ hz, Dims d, const int *__restrict__ offsets,
+              const int *__restrict__ place, int *__restrict__ order) {
+  Voxel v;
+  if (!voxel_of(d, v)) return;
+  const long b = bucket_of(d, hx[v.i], hy[v.i], hz[v.i]);
+  if (b >= 0) order[offsets[b] + place[v.i]] = (int)v.i;
 }
 
 // Buckets of up to kSmallBucket sources are insertion-sorted by one thread
@@ -285,149 +280,312 @@ AW_D void block_radix_sort(int *__restrict__ order, int *__restrict__ tmp, int s
   __syncthreads();
 }
 
-// Sorts every bucket by source index; with wts, then writes the eight corner
-// weights of the source at every sorted position, once per sort: the gathers
-// of every image splatted by the same h read them instead of the source's h
-// and the weight arithmetic. One CTA per 256 buckets; tmp (the scatter's
-// cursors, dead by now) holds at least n ints.
+// Sorts every bucket by source index. One CTA per 256 buckets; tmp (the
+// sources' places, dead by now) holds at least n + 2 ints.
 __global__ void __launch_bounds__(kSortThreads)
     k_bucket_sort(const int *__restrict__ offsets, int *__restrict__ order, int *__restrict__ tmp,
-                  long next, const float *__restrict__ hx, const float *__restrict__ hy,
-                  const float *__restrict__ hz, float *__restrict__ wts) {
+                  long next, long n) {
   __shared__ SortShared sh;
-  if (threadIdx.x == 0) sh.nlarge = 0;
-  __syncthreads();
+  // the sums' queue (tmp's first n places, then its count and the blocks
+  // done with it) starts empty
+  if (blockIdx.x == 0 && threadIdx.x < 2) tmp[n + threadIdx.x] = 0;
   const long b = (long)blockIdx.x * kSortThreads + threadIdx.x;
-  if (b < next) {
-    const int s = offsets[b], e = offsets[b + 1];
-    if (e - s <= kSmallBucket) {
-      for (int i = s + 1; i < e; ++i) {
-        const int key = order[i];
-        int j = i - 1;
-        while (j >= s && order[j] > key) {
-          order[j + 1] = order[j];
-          --j;
-        }
-        order[j + 1] = key;
+  const int s = b < next ? offsets[b] : 0, e = b < next ? offsets[b + 1] : 0;
+  const bool large = e - s > kSmallBucket;
+  if (!large) {
+    for (int i = s + 1; i < e; ++i) {
+      const int key = order[i];
+      int j = i - 1;
+      while (j >= s && order[j] > key) {
+        order[j + 1] = order[j];
+        --j;
       }
-      if (wts)
-        for (int i = s; i < e; ++i) store_weights(order, i, hx, hy, hz, wts);
-    } else {
-      sh.large[atomicAdd(&sh.nlarge, 1)] = threadIdx.x;
+      order[j + 1] = key;
     }
   }
+  if (!__syncthreads_or(large)) return;
+  if (threadIdx.x == 0) sh.nlarge = 0;
+  __syncthreads();
+  if (large) sh.large[atomicAdd(&sh.nlarge, 1)] = threadIdx.x;
   __syncthreads();
   const int nl = sh.nlarge;
   for (int q = 0; q < nl; ++q) {
     const long bb = (long)blockIdx.x * kSortThreads + sh.large[q];
-    const int s = offsets[bb], e = offsets[bb + 1];
-    block_radix_sort(order, tmp, s, e, sh);
-    if (wts)
-      for (int i = s + threadIdx.x; i < e; i += kSortThreads) store_weights(order, i, hx, hy, hz, wts);
+    block_radix_sort(order, tmp, offsets[bb], offsets[bb + 1], sh);
   }
 }
 
-// every destination merges its eight candidate buckets in source order (the
-// order forwardApply adds them). Buckets (dx = 1, dx = 0) of one (dy, dz) are
-// adjacent: three offsets bound both.
+// A source's eight contributions, corner weight times value, at its place in
+// the order: one plane of n per corner (dx + 2 dy + 4 dz), so that the sums
+// of neighbouring destinations, which want the same corner of neighbouring
+// places, read consecutive values, one load a contribution and none that
+// waits for the source's index.
+__global__ void __launch_bounds__(256)
+    k_products(const int *__restrict__ order, const int *__restrict__ total, long n,
+               const float *__restrict__ img, const float *__restrict__ hx,
+               const float *__restrict__ hy, const float *__restrict__ hz,
+               float *__restrict__ prod) {
+  const int p = blockIdx.x * 256 + threadIdx.x;
+  if (p >= *total) return;
+  const int m = order[p];
+  const Fractions f = fractions_of(__ldg(hx + m), __ldg(hy + m), __ldg(hz + m));
+  const float v = __ldg(img + m);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    prod[k * n + p] = fmul(corner_weight(f, k & 1, (k >> 1) & 1, (k >> 2) & 1), v);
+}
+
+// Every destination sums its contributions in source order, the order
+// forwardApply adds them. Its candidates lie in eight buckets: the cell
+// v - (dx, dy, dz) contributes its corner (dx, dy, dz). Buckets dx = 1 and
+// dx = 0 of one (dy, dz) are adjacent in the order, so three offsets bound
+// both, and four such ranges hold all candidates, eight on average.
 //
-// Fast path: the bucket of corner (dx, dy, dz) is the cell v - (dx, dy, dz),
-// so its sources usually precede those of every corner with a smaller
-// dx + 2 dy + 4 dz. The four (dy, dz) ranges are walked in that order
-// (dz = 1 first, then dy = 1; dx = 1 before dx = 0 inside each); when every
-// source index exceeds the one before it, this walk is the merged order and
-// the sum is complete. A source out of order (a folding or strongly
-// compressing map) sends the destination to the general eight-way merge,
-// which starts the sum again. (Fetching all candidates up front and merging
-// them in registers measured slower: the 16-way selection costs more issue
-// slots than the dependent loads it saves.)
-template <bool PRE>
-__global__ void __launch_bounds__(kRowThreads)
-    k_gather(const float *__restrict__ img, const float *__restrict__ hx,
-             const float *__restrict__ hy, const float *__restrict__ hz, Dims d,
-             const int *__restrict__ offsets, const int *__restrict__ order,
-             const float *__restrict__ wts, float *__restrict__ out, float bg) {
-  Voxel v;
-  if (!voxel_of(d, v)) return;
-  int pos[8], end[8], cur[8];
-  const long sy = d.nx + 1, sz = (long)(d.nx + 1) * (d.ny + 1);
-  // bucket k = (dz, dy, dx) bits; source in bucket b contributes corner
-  // (dx, dy, dz) to this voxel
+// Most destinations meet their sources in order when the ranges are walked
+// from (dy, dz) = (1, 1) down to (0, 0): up to kPer candidates of each range
+// are fetched at once, their indices and their products (k_products), and
+// where the indices rise, the products are added as they come. The others, 14 % of
+// them on a map with half a voxel of relief and 35 % on a compressing one,
+// lie scattered over nearly every warp: k_gather only queues them, and
+// k_gather_queued takes them one per thread, so that whole warps do the
+// ordering instead of a few lanes of each. There each pair of candidates out
+// of order moves its two ranks apart, kept four bits each in two words (a
+// compare and an addition a pair, without divergence), and the products go
+// to shared memory by rank and are added from there. A destination with more
+// than kMore candidates beyond the first kPer of their ranges merges its
+// eight sorted buckets one source at a time.
+constexpr int kGatherThreads = 256, kQueuedThreads = 128;
+constexpr int kPer = 3, kMore = 4, kFirst = 4 * kPer, kSlots = kFirst + kMore;
+static_assert(kSlots == 16, "ranks of four bits in two words");
+
+struct GatherArgs {
+  Dims d;
+  long n;
+  IdxDiv byNx, byNy;
+  const float *img, *hx, *hy, *hz;
+  const float *prod;  // PRE: the products; else they are formed here
+  const int *offsets, *order;
+  int *queue;  // n destinations, then their count and the blocks done with it
+  float *out;
+  float bg;
+};
+
+// the four candidate ranges of a destination, each [beg, mid) at dx = 1 and
+// [mid, end) at dx = 0
+struct Ranges {
+  int beg[4], mid[4], end[4];
+};
+AW_D Ranges ranges_of(const GatherArgs &a, int i) {
+  const int row = a.byNx.div(i), x = i - row * a.d.nx, z = a.byNy.div(row), y = row - z * a.d.ny;
+  const int sy = a.d.nx + 1, sz = sy * (a.d.ny + 1);  // buckets fit 31 bits
+  Ranges q;
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int dy = r & 1, dz = r >> 1;
-    const long b1 = (long)(v.z - dz + 1) * sz + (long)(v.y - dy + 1) * sy + v.x;  // dx = 1
-    const int o0 = __ldg(offsets + b1), o1 = __ldg(offsets + b1 + 1), o2 = __ldg(offsets + b1 + 2);
-    pos[2 * r + 1] = o0;
-    end[2 * r + 1] = o1;
-    pos[2 * r] = o1;
-    end[2 * r] = o2;
+    const int *o = a.offsets + ((z - dz + 1) * sz + (y - dy + 1) * sy + x);
+    q.beg[r] = __ldg(o);
+    q.mid[r] = __ldg(o + 1);
+    q.end[r] = __ldg(o + 2);
   }
-  float acc = bg;
-  int prev = -1;
-  bool ordered = true;
+  return q;
+}
+// the product of source m at place p of the order; corner k = dx + 2 dy + 4 dz
+template <bool PRE>
+AW_D float contribution(const GatherArgs &a, int p, int m, int k) {
+  if (PRE) return __ldg(a.prod + ((long)k * a.n + p));
+  return fmul(corner_weight(fractions_of(__ldg(a.hx + m), __ldg(a.hy + m), __ldg(a.hz + m)), k & 1,
+                            (k >> 1) & 1, (k >> 2) & 1),
+              __ldg(a.img + m));
+}
+
+// any number of candidates: the smallest head of the eight sorted buckets
+template <bool PRE>
+__device__ __noinline__ float sum_by_merging(const GatherArgs &a, const Ranges &q) {
+  int pos[8], cur[8];
 #pragma unroll
-  for (int r = 3; r >= 0; --r) {
-    const int dy = r & 1, dz = r >> 1;
-    for (int p = pos[2 * r + 1]; ordered && p < end[2 * r]; ++p) {
-      const int m = __ldg(order + p);
-      if (m <= prev) {
-        ordered = false;
-        break;
-      }
-      prev = m;
-      const int dx = p < end[2 * r + 1] ? 1 : 0;
-      const float w = PRE ? __ldg(wts + (long)p * 8 + (dx + 2 * dy + 4 * dz))
-                          : corner_weight(hx[m], hy[m], hz[m], dx, dy, dz);
-      acc = fadd(acc, fmul(w, img[m]));
-    }
+  for (int k = 0; k < 8; ++k) {
+    pos[k] = (k & 1) ? q.beg[k >> 1] : q.mid[k >> 1];
+    cur[k] = pos[k] < ((k & 1) ? q.mid[k >> 1] : q.end[k >> 1]) ? a.order[pos[k]] : INT_MAX;
   }
-  if (ordered) {
-    out[v.i] = acc;
-    return;
-  }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) cur[k] = pos[k] < end[k] ? order[pos[k]] : INT_MAX;
-  acc = bg;
+  float acc = a.bg;
   while (true) {
-    int m = INT_MAX, sel = -1;
+    int m = INT_MAX, sel = -1, at = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k)
       if (cur[k] < m) {
         m = cur[k];
         sel = k;
+        at = pos[k];
       }
-    if (sel < 0) break;
-    int at = 0;
+    if (sel < 0) return acc;
+    acc = fadd(acc, contribution<PRE>(a, at, m, sel));
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-      if (k == sel) at = pos[k];
-    const float w = PRE ? __ldg(wts + (long)at * 8 + sel)
-                        : corner_weight(hx[m], hy[m], hz[m], sel & 1, (sel >> 1) & 1,
-                                        (sel >> 2) & 1);
-    acc = fadd(acc, fmul(w, img[m]));
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
       if (k == sel) {
         ++pos[k];
-        cur[k] = pos[k] < end[k] ? order[pos[k]] : INT_MAX;
+        cur[k] = pos[k] < ((k & 1) ? q.mid[k >> 1] : q.end[k >> 1]) ? a.order[pos[k]] : INT_MAX;
       }
+  }
+}
+
+// candidate c of the first kPer of every range, in the walk's order: its
+// range, and its index or INT_MAX
+AW_D constexpr int range_of(int c) { return 3 - c / kPer; }
+AW_D void first_candidates(const GatherArgs &a, const Ranges &q, int *m) {
+#pragma unroll
+  for (int r = 3; r >= 0; --r) {
+    const int *o = a.order + q.beg[r];
+    const int len = q.end[r] - q.beg[r];
+#pragma unroll
+    for (int c = 0; c < kPer; ++c) m[(3 - r) * kPer + c] = c < len ? __ldg(o + c) : INT_MAX;
+  }
+}
+// their products (0 for none)
+template <bool PRE>
+AW_D void first_products(const GatherArgs &a, const Ranges &q, const int *m, float *pr) {
+#pragma unroll
+  for (int r = 3; r >= 0; --r) {
+    // corner dx = 0 of range r, and dx = 1 one plane on
+    const float *w0 = PRE ? a.prod + ((long)(2 * r) * a.n + q.beg[r]) : nullptr;
+    const float *w1 = PRE ? w0 + a.n : nullptr;
+    const int len = q.end[r] - q.beg[r], ones = q.mid[r] - q.beg[r];
+#pragma unroll
+    for (int c = 0; c < kPer; ++c) {
+      const int i = (3 - r) * kPer + c;
+      if (PRE)
+        pr[i] = c < len ? __ldg((c < ones ? w1 : w0) + c) : 0.f;
+      else
+        pr[i] = c < len ? contribution<PRE>(a, q.beg[r] + c, m[i], 2 * r + (c < ones ? 1 : 0)) : 0.f;
     }
   }
-  out[v.i] = acc;
+}
+
+template <bool PRE>
+__global__ void __launch_bounds__(kGatherThreads) k_gather(const __grid_constant__ GatherArgs a) {
+  const int i = blockIdx.x * kGatherThreads + threadIdx.x;
+  bool later = false;
+  if (i < a.n) {
+    const Ranges q = ranges_of(a, i);
+    int m[kFirst], top = -1;
+    float pr[kFirst];
+    first_candidates(a, q, m);
+    if (PRE) first_products<PRE>(a, q, m, pr);
+#pragma unroll
+    for (int r = 3; r >= 0; --r) {
+      const int *c = m + (3 - r) * kPer;
+      static_assert(kPer == 3, "a range's largest index");
+      const int len = q.end[r] - q.beg[r];
+      later = later || len > kPer || c[0] < top || c[1] < c[0] || c[2] < c[1];
+      top = max(top, len > 2 ? c[2] : (len > 1 ? c[1] : (len > 0 ? c[0] : -1)));
+    }
+    if (!later) {
+      float acc = a.bg;
+      if (!PRE) first_products<PRE>(a, q, m, pr);
+#pragma unroll
+      for (int c = 0; c < kFirst; ++c)
+        if (m[c] != INT_MAX) acc = fadd(acc, pr[c]);
+      a.out[i] = acc;
+    }
+  }
+  const unsigned who = __ballot_sync(0xffffffffu, later);
+  if (!who) return;
+  const int lane = threadIdx.x & 31;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(a.queue + a.n, __popc(who));
+  at = __shfl_sync(0xffffffffu, at, 0);
+  if (later) a.queue[at + __popc(who & ((1u << lane) - 1u))] = i;
+}
+
+// entries i < j of the walk: out of order, their ranks move apart
+AW_D void rank_pair(unsigned (&rk)[2], const int *m, int i, int j) {
+  if (m[j] >= m[i]) return;
+  if (i / 8 == j / 8) {
+    rk[i / 8] += (1u << (4 * (i % 8))) - (1u << (4 * (j % 8)));
+  } else {
+    rk[i / 8] += 1u << (4 * (i % 8));
+    rk[j / 8] -= 1u << (4 * (j % 8));
+  }
+}
+
+// the queued destinations, one per thread; the last block to finish empties
+// the queue for the next image splatted by the same map
+template <bool PRE>
+__global__ void __launch_bounds__(kQueuedThreads) k_gather_queued(const __grid_constant__ GatherArgs a) {
+  __shared__ float byrank[kSlots][kQueuedThreads];
+  const int tid = threadIdx.x, count = *(volatile int *)(a.queue + a.n);
+  for (int t = blockIdx.x * kQueuedThreads + tid; t < count; t += gridDim.x * kQueuedThreads) {
+    const int i = a.queue[t];
+    const Ranges q = ranges_of(a, i);
+    int more = 0, total = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int len = q.end[r] - q.beg[r];
+      more += max(len - kPer, 0);
+      total += len;
+    }
+    if (more > kMore) {
+      a.out[i] = sum_by_merging<PRE>(a, q);
+      continue;
+    }
+    int m[kSlots];
+    float pr[kSlots];
+    first_candidates(a, q, m);
+    first_products<PRE>(a, q, m, pr);
+    // ranks start as the walk's own order; the absent sort behind
+    unsigned rk[2] = {0x76543210u, 0xfedcba98u};
+#pragma unroll
+    for (int j = 1; j < kFirst; ++j)
+#pragma unroll
+      for (int c = 0; c < j; ++c) rank_pair(rk, m, c, j);
+    if (more) {
+      // the c-th candidate past the first kPer of its range, ranges in the
+      // walk's order
+#pragma unroll
+      for (int c = 0; c < kMore; ++c) {
+        int left = c, p = -1, k = 0;
+#pragma unroll
+        for (int r = 3; r >= 0; --r) {
+          const int over = max(q.end[r] - q.beg[r] - kPer, 0);
+          if (p < 0 && left < over) {
+            p = q.beg[r] + kPer + left;
+            k = (p < q.mid[r] ? 1 : 0) + 2 * r;
+          }
+          left -= over;
+        }
+        m[kFirst + c] = p >= 0 ? __ldg(a.order + p) : INT_MAX;
+        pr[kFirst + c] = p >= 0 ? contribution<PRE>(a, p, m[kFirst + c], k) : 0.f;
+      }
+#pragma unroll
+      for (int j = kFirst; j < kSlots; ++j)
+#pragma unroll
+        for (int c = 0; c < j; ++c) rank_pair(rk, m, c, j);
+#pragma unroll
+      for (int c = kFirst; c < kSlots; ++c) byrank[(rk[1] >> (4 * (c % 8))) & 15u][tid] = pr[c];
+    }
+#pragma unroll
+    for (int c = 0; c < kFirst; ++c) byrank[(rk[c / 8] >> (4 * (c % 8))) & 15u][tid] = pr[c];
+    float acc = a.bg;
+    for (int c = 0; c < total; ++c) acc = fadd(acc, byrank[c][tid]);
+    a.out[i] = acc;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    unsigned *done = reinterpret_cast<unsigned *>(a.queue + a.n + 1);
+    if (atomicInc(done, gridDim.x - 1) == gridDim.x - 1) a.queue[a.n] = 0;
+  }
 }
 
 }  // namespace
 
-size_t splat_scratch_bytes(const Dims &d, bool weights) {
+size_t splat_scratch_bytes(const Dims &d, bool products) {
   const long next = (long)(d.nx + 1) * (d.ny + 1) * (d.nz + 1);
   const long nb = (next + kScanBlock - 1) / kScanBlock;
   return align256(sizeof(int) * (next + 1)) + align256(sizeof(int) * next) +
          align256(sizeof(int) * d.n()) + align256(sizeof(int) * nb) +
-         (weights ? align256(sizeof(float) * 8 * d.n()) : 0);
+         (products ? align256(sizeof(float) * 8 * d.n()) : 0);
 }
 
-void splat_work_bind(SplatWork *w, const Dims &d, void *scratch, bool weights) {
+void splat_work_bind(SplatWork *w, const Dims &d, void *scratch, bool products) {
   char *p = static_cast<char *>(scratch);
   w->d = d;
   w->next = (long)(d.nx + 1) * (d.ny + 1) * (d.nz + 1);
@@ -440,7 +598,7 @@ void splat_work_bind(SplatWork *w, const Dims &d, void *scratch, bool weights) {
   p += align256(sizeof(int) * d.n());
   w->blocksums = reinterpret_cast<int *>(p);
   p += align256(sizeof(int) * w->nblocks);
-  w->wts = weights ? reinterpret_cast<float *>(p) : nullptr;
+  w->prod = products ? reinterpret_cast<float *>(p) : nullptr;
 }
 
 cudaError_t splat_sort(const SplatWork &w, const float *hx, const float *hy, const float *hz,
@@ -448,26 +606,33 @@ cudaError_t splat_sort(const SplatWork &w, const float *hx, const float *hy, con
   const Dims d = w.d;
   cudaError_t e;
   if ((e = cudaMemsetAsync(w.offsets, 0, sizeof(int) * (w.next + 1), s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(w.cursor, 0, sizeof(int) * w.next, s)) != cudaSuccess) return e;
-  k_count<<<row_grid(d), kRowThreads, 0, s>>>(hx, hy, hz, d, w.offsets);
+  k_count<<<row_grid(d), kRowThreads, 0, s>>>(hx, hy, hz, d, w.offsets, w.cursor);
   k_scan_reduce<<<w.nblocks, kScanThreads, 0, s>>>(w.offsets, w.next, w.blocksums);
   k_scan_blocksums<<<1, kScanThreads, 0, s>>>(w.blocksums, w.nblocks);
   k_scan_apply<<<w.nblocks, kScanThreads, 0, s>>>(w.offsets, w.next, w.blocksums);
   k_scatter<<<row_grid(d), kRowThreads, 0, s>>>(hx, hy, hz, d, w.offsets, w.cursor, w.order);
   k_bucket_sort<<<(int)((w.next + kSortThreads - 1) / kSortThreads), kSortThreads, 0, s>>>(
-      w.offsets, w.order, w.cursor, w.next, hx, hy, hz, w.wts);
+      w.offsets, w.order, w.cursor, w.next, d.n());
   return cudaGetLastError();
 }
 
 cudaError_t splat_gather(const SplatWork &w, const float *img, const float *hx, const float *hy,
                          const float *hz, float *out, float bg, cudaStream_t s) {
   const Dims d = w.d;
-  if (w.wts)
-    k_gather<true><<<row_grid(d), kRowThreads, 0, s>>>(img, hx, hy, hz, d, w.offsets, w.order,
-                                                       w.wts, out, bg);
-  else
-    k_gather<false><<<row_grid(d), kRowThreads, 0, s>>>(img, hx, hy, hz, d, w.offsets, w.order,
-                                                        nullptr, out, bg);
+  const GatherArgs a{d,  d.n(), make_idxdiv((uint32_t)d.nx), make_idxdiv((uint32_t)d.ny), img, hx, hy,
+                     hz, w.prod, w.offsets, w.order, w.cursor, out, bg};
+  const unsigned grid = (unsigned)((d.n() + kGatherThreads - 1) / kGatherThreads);
+  // seven blocks an SM, or one thread per destination
+  const unsigned queued = (unsigned)std::min<long>((d.n() + kQueuedThreads - 1) / kQueuedThreads, 7 * 148);
+  if (w.prod) {
+    k_products<<<(unsigned)((d.n() + 255) / 256), 256, 0, s>>>(w.order, w.offsets + w.next, d.n(), img,
+                                                               hx, hy, hz, w.prod);
+    k_gather<true><<<grid, kGatherThreads, 0, s>>>(a);
+    k_gather_queued<true><<<queued, kQueuedThreads, 0, s>>>(a);
+  } else {
+    k_gather<false><<<grid, kGatherThreads, 0, s>>>(a);
+    k_gather_queued<false><<<queued, kQueuedThreads, 0, s>>>(a);
+  }
   return cudaGetLastError();
 }
 

@@ -23,18 +23,19 @@ struct SplatWork {
   Dims d;
   long next;        // (nx+1)(ny+1)(nz+1)
   int *offsets;     // next + 1: bucket counts, then exclusive offsets
-  int *cursor;      // next: scatter cursors
+  int *cursor;      // next: each source's place in its bucket, the sort's scratch, the sums' queue
   int *order;       // n: source indices grouped by bucket
   int *blocksums;   // scan partials
   int nblocks;
-  float *wts;       // 8n or null: the corner weights of the source at each sorted position
+  float *prod;      // 8n or null: per corner, weight times value of the source at each position of order
 };
 
-// bytes of device scratch one splat of grid d needs; weights: room for the
-// corner weights the sort can precompute (32 bytes per voxel)
-size_t splat_scratch_bytes(const Dims &d, bool weights = true);
+// bytes of device scratch one splat of grid d needs; products: room for the
+// sources' eight contributions (32 bytes per voxel), which the sums otherwise
+// form themselves
+size_t splat_scratch_bytes(const Dims &d, bool products = true);
 // lays out a SplatWork inside caller-provided device memory (256-aligned)
-void splat_work_bind(SplatWork *w, const Dims &d, void *scratch, bool weights = true);
+void splat_work_bind(SplatWork *w, const Dims &d, void *scratch, bool products = true);
 
 // out = splat of img by h (three planes), background bg; stream-ordered
 cudaError_t splat(const SplatWork &w, const float *img, const float *hx, const float *hy,
