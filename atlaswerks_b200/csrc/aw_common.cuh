@@ -12,6 +12,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <utility>
+
 #define AW_HD __host__ __device__ __forceinline__
 #define AW_D __device__ __forceinline__
 
@@ -46,6 +48,31 @@ AW_D bool voxel_of(const Dims &d, Voxel &v) {
   v.z = blockIdx.z;
   v.i = ((long)v.z * d.ny + v.y) * d.nx + v.x;
   return v.x < d.nx;
+}
+
+// Programmatic dependent launch: a kernel launched by launch_early may begin
+// while the kernel before it on the stream is still running, once every block
+// of that one has called dependents_may_start (or has ended). It fetches its
+// constant tables and sets up its barriers, then waits in
+// wait_for_predecessors, before the first access to anything an earlier
+// kernel writes or reads, until that kernel has completed. Both calls do
+// nothing in a kernel launched in the ordinary way.
+AW_D void wait_for_predecessors() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+AW_D void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem,
+                         cudaStream_t s, A &&...args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 // n / d for 0 <= n < 2^31 by multiply and shift (round-up method)

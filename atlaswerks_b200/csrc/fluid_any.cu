@@ -372,6 +372,7 @@ __global__ void __launch_bounds__(kXYMaxThreads) k_any_xy_fwd(const __grid_const
   copy_table(twy, p.y.tw, p.y.n);
   for (int i = threadIdx.x; i < p.ncol; i += blockDim.x) cols[i] = __ldg(p.cols + i);
   if (threadIdx.x == 0 && (H * p.pitch & 1)) S[H * p.pitch] = make_float2(0.f, 0.f);
+  wait_for_predecessors();
   produce(p, src, S, z, comp, 0, H);
   __syncthreads();
   // x and y stages by one loop, so that they share their code. Before the
@@ -437,6 +438,7 @@ __global__ void __launch_bounds__(kXYMaxThreads) k_any_xy_fwd(const __grid_const
     // the first two pairs are their own (ky = 0, then ny / 2 of an even ny)
     S[w2 != w ? at(w2) : (i == 0 ? p.d.nx : p.pad1)] = CN;
   }
+  dependents_may_start();
   fence_async_smem();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -455,6 +457,7 @@ __global__ void __launch_bounds__(kXYMaxThreads) k_any_xy_inv(const __grid_const
   copy_table(twx, p.x.tw, p.x.n);
   copy_table(twy, p.y.tw, p.y.n);
   for (int i = threadIdx.x; i < p.ncol; i += blockDim.x) cols[i] = __ldg(p.cols + i);
+  wait_for_predecessors();
   if (threadIdx.x == 0) {
     const uint32_t bytes = (uint32_t)(sizeof(float2) * p.slab);
     mbar_init(&mbar, 1);
@@ -543,6 +546,7 @@ __global__ void __launch_bounds__(kSplitMaxThreads, 2) k_any_x_fwd(const __grid_
   float2 *S = sm, *twx = S + ((p.P * p.pitch + 1) & ~1);
   copy_table(twx, p.x.tw, p.x.n);
   if (threadIdx.x == 0 && whole > places) S[places] = make_float2(0.f, 0.f);
+  wait_for_predecessors();
   produce(p, src, S, z, comp, p0, np);
   __syncthreads();
   const IdxDiv byL = np == p.P ? p.byP : p.byLast;
@@ -566,6 +570,7 @@ __global__ void __launch_bounds__(kSplitMaxThreads, 2) k_any_x_inv(const __grid_
   const int z = blockIdx.x, comp = blockIdx.y, p0 = blockIdx.z * p.P, np = min(p.P, p.H - p0);
   float2 *S = sm, *twx = S + ((p.P * p.pitch + 1) & ~1);
   copy_table(twx, p.x.tw, p.x.n);
+  wait_for_predecessors();
   if (threadIdx.x == 0) {
     const uint32_t bytes = (uint32_t)(sizeof(float2) * ((np * p.pitch + 1) & ~1));
     mbar_init(&mbar, 1);
@@ -598,6 +603,7 @@ __global__ void __launch_bounds__(kSplitMaxThreads, 2) k_any_y(const __grid_cons
   const int A = (int)(ab & 0xffffu), B = (int)(ab >> 16);
   const int rows = (int)blockDim.x >> lq, r0 = (int)threadIdx.x >> lq;
   const AtTile at{ny, Q, lq};
+  wait_for_predecessors();
   if (SIGN < 0) {
 #pragma unroll 4
     for (int l = r0; l < H; l += rows) {
@@ -713,6 +719,7 @@ __global__ void __launch_bounds__(kZMaxThreads, 4) k_any_z(const __grid_constant
   const AtTile at{nz, Q, lq};
   const AnyStage first = p.z.st[0];
   const int rows = (int)blockDim.x >> lq, r0 = (int)threadIdx.x >> lq;
+  wait_for_predecessors();
   __syncthreads();
   // the first radix straight from HBM (a single stage: a plain copy)
   const bool direct = ns > 1 && first.R <= kZRadix;
@@ -773,6 +780,7 @@ __global__ void __launch_bounds__(kZMaxThreads, 4) k_any_z(const __grid_constant
       solve(lz[w], t[0], t[tile], t[2 * tile]);
     }
   }
+  dependents_may_start();
   __syncthreads();
 #pragma unroll 1
   for (int s = s1 - 1; s >= s0; --s) {
@@ -1045,31 +1053,30 @@ void any_set_split(AnyPlan *p, int P, int Q, size_t maxsm) {
 template <class Src>
 cudaError_t any_forward(const AnyPlan &p, const Src &src, bool split, cudaStream_t s) {
   const AnyXY &a = p.xy;
-  if (!split) {
-    k_any_xy_fwd<Src><<<dim3(a.d.nz, 3), p.threads_xy, p.smem_xy, s>>>(a, src);
-    return cudaGetLastError();
-  }
-  k_any_x_fwd<Src><<<dim3(a.d.nz, 3, (a.H + a.P - 1) / a.P), 256, p.smem_x, s>>>(a, src);
-  k_any_y<-1><<<dim3(a.d.nz, 3, (a.ncol + a.Q - 1) / a.Q), p.threads_y, p.smem_y, s>>>(a);
-  return cudaGetLastError();
+  if (!split)
+    return launch_early(k_any_xy_fwd<Src>, dim3(a.d.nz, 3), p.threads_xy, p.smem_xy, s, a, src);
+  const cudaError_t e = launch_early(k_any_x_fwd<Src>, dim3(a.d.nz, 3, (a.H + a.P - 1) / a.P), 256,
+                                     p.smem_x, s, a, src);
+  if (e != cudaSuccess) return e;
+  return launch_early(k_any_y<-1>, dim3(a.d.nz, 3, (a.ncol + a.Q - 1) / a.Q), p.threads_y, p.smem_y,
+                      s, a);
 }
 
 template <class Dst>
 cudaError_t any_inverse(const AnyPlan &p, const Dst &dst, bool split, cudaStream_t s) {
   const AnyXY &a = p.xy;
-  if (!split) {
-    k_any_xy_inv<Dst><<<dim3(a.d.nz, 3), p.threads_xy, p.smem_xy, s>>>(a, dst);
-    return cudaGetLastError();
-  }
-  k_any_y<+1><<<dim3(a.d.nz, 3, (a.ncol + a.Q - 1) / a.Q), p.threads_y, p.smem_y, s>>>(a);
-  k_any_x_inv<Dst><<<dim3(a.d.nz, 3, (a.H + a.P - 1) / a.P), 256, p.smem_x, s>>>(a, dst);
-  return cudaGetLastError();
+  if (!split)
+    return launch_early(k_any_xy_inv<Dst>, dim3(a.d.nz, 3), p.threads_xy, p.smem_xy, s, a, dst);
+  const cudaError_t e = launch_early(k_any_y<+1>, dim3(a.d.nz, 3, (a.ncol + a.Q - 1) / a.Q),
+                                     p.threads_y, p.smem_y, s, a);
+  if (e != cudaSuccess) return e;
+  return launch_early(k_any_x_inv<Dst>, dim3(a.d.nz, 3, (a.H + a.P - 1) / a.P), 256, p.smem_x, s, a,
+                      dst);
 }
 
 cudaError_t any_solve(const AnyPlan &p, int inverse, cudaStream_t s) {
   const int grid = (int)((p.z.pcols + p.z.q - 1) / p.z.q);
-  k_any_z<<<grid, p.threads_z, p.smem_z, s>>>(p.z, inverse);
-  return cudaGetLastError();
+  return launch_early(k_any_z, dim3(grid), p.threads_z, p.smem_z, s, p.z, inverse);
 }
 
 // the kernels of a plan and the shared memory each needs

@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(kXYThreads, (XYShape<NX, NY>::ctas()))
   const int z = blockIdx.x, comp = blockIdx.y;
   const SmemTw twx = copy_twiddles<NX, NY>(sm, p);
   const SmemTw twy{twx.p + NX};
+  wait_for_predecessors();
   __syncthreads();
 
   // ---- x: row pairs (y0, y0+1) as one complex line, exchanged in place ----
@@ -199,6 +200,7 @@ __global__ void __launch_bounds__(kXYThreads, (XYShape<NX, NY>::ctas()))
   }
 
   // ---- store the slab: one bulk copy shared -> HBM -----------------------
+  dependents_may_start();
   fence_async_smem();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -314,6 +316,7 @@ AW_D void inv_x_pass(float2 *C, const SmemTw &tw, int warp, int lane, const Out 
 template <int NX, int NY>
 AW_D bool load_slab(float2 *C, uint64_t *mbar, const FluidPlan &p, int z, int comp) {
   using S = XYShape<NX, NY>;
+  wait_for_predecessors();
   if (threadIdx.x == 0) {
     const uint32_t bytes = (uint32_t)(sizeof(float2) * NY * S::NXH);
     mbar_init(mbar, 1);
@@ -502,6 +505,7 @@ __global__ void __launch_bounds__(z_threads<NZ, Q>(), (NZ <= 128 ? 48 / Q : 16 /
   const int c = line / Q, q = line % Q;
   float2 *tile = TB + c * TILE;
   bool ok = true;
+  wait_for_predecessors();
   if constexpr (TMA) {
     if (threadIdx.x == 0) {
       for (int cc = 0; cc < 3; ++cc) mbar_init(&mbar[cc], 1);
@@ -543,6 +547,7 @@ __global__ void __launch_bounds__(z_threads<NZ, Q>(), (NZ <= 128 ? 48 / Q : 16 /
   }
   __syncthreads();
 
+  dependents_may_start();
 #pragma unroll
   for (int j = 0; j < E; ++j) v[j] = tile[zt<Q>(t + T * j, q)];
   line_fft<NZ, +1>(v, t, [tile, q](int m) { return tile + zt<Q>(m, q); }, tw);
@@ -627,24 +632,28 @@ cudaError_t fast_configure(const FluidPlan &p) {
 
 template <class Src>
 cudaError_t fast_xy_forward(const FluidPlan &p, const Src &src, cudaStream_t s) {
+  cudaError_t e = cudaErrorInvalidValue;
   dispatch_n(p.d.nx, [&](auto X) {
     dispatch_n(p.d.ny, [&](auto Y) {
       constexpr int NX = decltype(X)::value, NY = decltype(Y)::value;
-      k_xy_fwd_fast<NX, NY, Src><<<dim3(p.d.nz, 3), kXYThreads, p.fast_smem_xy, s>>>(p, src);
+      e = launch_early(k_xy_fwd_fast<NX, NY, Src>, dim3(p.d.nz, 3), kXYThreads, p.fast_smem_xy, s, p,
+                       src);
     });
   });
-  return cudaGetLastError();
+  return e;
 }
 
 template <class Dst>
 cudaError_t fast_xy_inverse(const FluidPlan &p, const Dst &dst, cudaStream_t s) {
+  cudaError_t e = cudaErrorInvalidValue;
   dispatch_n(p.d.nx, [&](auto X) {
     dispatch_n(p.d.ny, [&](auto Y) {
       constexpr int NX = decltype(X)::value, NY = decltype(Y)::value;
-      k_xy_inv_fast<NX, NY, Dst><<<dim3(p.d.nz, 3), kXYThreads, p.fast_smem_xy, s>>>(p, dst);
+      e = launch_early(k_xy_inv_fast<NX, NY, Dst>, dim3(p.d.nz, 3), kXYThreads, p.fast_smem_xy, s, p,
+                       dst);
     });
   });
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t fast_xy_inverse_compose(const FluidPlan &p, const ComposeArgs &a, cudaStream_t s) {
@@ -665,19 +674,23 @@ cudaError_t fast_z_solve(const FluidPlan &p, int inverse, cudaStream_t s) {
   const long ncols = (long)p.d.ny * p.nxh;
   const int q = p.fast_kq == 8 ? 8 : 16;
   const int grid = (int)((ncols + q - 1) / q);
+  cudaError_t e = cudaErrorInvalidValue;
   dispatch_n(p.d.nz, [&](auto Z) {
     constexpr int NZ = decltype(Z)::value;
     const size_t sm = fast_z_smem(NZ, q);
+    auto go = [&](auto kernel, unsigned threads) {
+      e = launch_early(kernel, dim3(grid), threads, sm, s, p, p.spec_map, inverse);
+    };
     if (q == 8 && p.fast_tma)
-      k_z_solve_fast<NZ, 8, true><<<grid, z_threads<NZ, 8>(), sm, s>>>(p, p.spec_map, inverse);
+      go(k_z_solve_fast<NZ, 8, true>, z_threads<NZ, 8>());
     else if (q == 8)
-      k_z_solve_fast<NZ, 8, false><<<grid, z_threads<NZ, 8>(), sm, s>>>(p, p.spec_map, inverse);
+      go(k_z_solve_fast<NZ, 8, false>, z_threads<NZ, 8>());
     else if (p.fast_tma)
-      k_z_solve_fast<NZ, 16, true><<<grid, z_threads<NZ, 16>(), sm, s>>>(p, p.spec_map, inverse);
+      go(k_z_solve_fast<NZ, 16, true>, z_threads<NZ, 16>());
     else
-      k_z_solve_fast<NZ, 16, false><<<grid, z_threads<NZ, 16>(), sm, s>>>(p, p.spec_map, inverse);
+      go(k_z_solve_fast<NZ, 16, false>, z_threads<NZ, 16>());
   });
-  return cudaGetLastError();
+  return e;
 }
 
 template cudaError_t fast_xy_forward<SrcField>(const FluidPlan &, const SrcField &, cudaStream_t);

@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(kRowThreads)
   const int x = blockIdx.x * kRowThreads + threadIdx.x;
   const int z = blockIdx.z;
   double e = 0.0;
+  dependents_may_start();
   if (x < d.nx) {
     const int y0 = blockIdx.y * kPrepRows;
     const int y1 = min(y0 + kPrepRows, d.ny);
