@@ -102,11 +102,27 @@ __global__ void __launch_bounds__(kXYThreads, (XYShape<NX, NY>::ctas()))
     static_assert(NLINES % 8 == 0 && NLINES % L == 0, "x-lines fill whole warps");
     constexpr int KU = (NXH + TX - 1) / TX;
     const int lw = lane / TX, t = lane % TX;
+    // few lines leave some warps without one: there all of them fetch (at
+    // 32 x 32 two of eight warps hold the 16 lines, eight row pairs each
+    // after the other)
+    constexpr bool kAllFetch = NX >= 32 && NLINES < kXYWarps * L;
+    if constexpr (kAllFetch) {
+      for (int g = warp; g < NLINES; g += kXYWarps) {
+        float2 u[NX / 32];
+        src.template row_pair<NX / 32, 32>(comp, lane, 2 * g, z, d, u);
+#pragma unroll
+        for (int j = 0; j < NX / 32; ++j) C[2 * g * NXH + lane + 32 * j] = u[j];
+      }
+      __syncthreads();
+    }
     for (int base = warp * L; base < NLINES; base += kXYWarps * L) {
       const int y0 = 2 * xline_pair<TX>(base + lw);
       float2 *row = C + y0 * NXH;
       float2 v[EX];
-      if constexpr (NX >= 32) {
+      if constexpr (kAllFetch) {
+#pragma unroll
+        for (int j = 0; j < EX; ++j) v[j] = row[t + TX * j];
+      } else if constexpr (NX >= 32) {
         // The warp's L row pairs, one at a time, with its 32 lanes on 32
         // consecutive x: every load is one 128-byte line (the line layout,
         // TX lanes of TX-strided x on each of L rows, would touch L lines
