@@ -753,11 +753,22 @@ __global__ void k_bias_partial(const bf16 *__restrict__ dy, long M, int N, float
     part[(long)blockIdx.x * N + threadIdx.x] = t;
   }
 }
-__global__ void k_bias_final(const float *__restrict__ part, int nb, int N, float *__restrict__ db) {
-  for (int n = threadIdx.x; n < N; n += blockDim.x) {
-    float t = 0.0f;
-    for (int b = 0; b < nb; ++b) t += part[(long)b * N + n];
-    db[n] = t;
+// one block per channel: strided sums, then the warp and block trees (the
+// same order on every run)
+__global__ void __launch_bounds__(kEw)
+    k_bias_final(const float *__restrict__ part, int nb, int N, float *__restrict__ db) {
+  const int n = blockIdx.x;
+  float t = 0.0f;
+  for (int b = threadIdx.x; b < nb; b += kEw) t += part[(long)b * N + n];
+  __shared__ float sh[kEw / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float u = 0.0f;
+    for (int w = 0; w < kEw / 32; ++w) u += sh[w];
+    db[n] = u;
   }
 }
 
@@ -833,11 +844,16 @@ struct DirectCfg {
   static_assert(CIN % 16 == 0 && COUT % 16 == 0 && COLS <= 256, "direct conv shape");
 };
 
-template <int CIN, int COUT, int ZT>
+// DGRAD: the data gradient of such a layer, the same sum with the taps
+// mirrored (dX[v] takes dY[v - off(tap)]), the weights' copy [ci][tap][co]
+// in the weights' place and the ReLU mask in the epilogue's. Taps run in
+// both from 0 to 26.
+template <int CIN, int COUT, int ZT, bool DGRAD>
 __global__ void __launch_bounds__(128)
     k_conv_direct(const __grid_constant__ CUtensorMap tmap, const bf16 *__restrict__ w,
-                  const float *__restrict__ bias, int relu, bf16 *__restrict__ out,
-                  float *__restrict__ outf, int D, int H, int W, int *status) {
+                  const float *__restrict__ bias, int relu, const bf16 *__restrict__ mask,
+                  bf16 *__restrict__ out, float *__restrict__ outf, int D, int H, int W,
+                  int *status) {
   using C = DirectCfg<CIN, COUT, ZT>;
   extern __shared__ __align__(1024) uint8_t smraw[];
   __shared__ uint64_t mbar[2];  // 0: input box landed, 1: MMAs done
@@ -892,7 +908,8 @@ __global__ void __launch_bounds__(128)
       for (int zz = 0; zz < ZT; ++zz) {
 #pragma unroll 1
         for (int tap = 0; tap < 27; ++tap) {
-          const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
+          const int at = DGRAD ? 26 - tap : tap;
+          const int dz = at / 9, dy = (at / 3) % 3, dx = at % 3;
           const uint32_t cell = (uint32_t)((((zz + dz) * 18 + dy) * 10 + dx) * 16);
 #pragma unroll
           for (int jp = 0; jp < C::NCH / 2; ++jp) {
@@ -919,13 +936,28 @@ __global__ void __launch_bounds__(128)
     for (int g = 0; g < COUT / 16; ++g) {
       float v[16];
       tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(zz * COUT + 16 * g), v);
-      float o[16];
+      float o[16], on[16];
+      if (DGRAD && mask) {  // 16-byte aligned (nn_conv_dgrad)
+        const uint4 *mp = reinterpret_cast<const uint4 *>(mask + m * COUT + 16 * g);
+        float lo[8], hi[8];
+        bf8_to_f(__ldg(mp), lo);
+        bf8_to_f(__ldg(mp + 1), hi);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          on[i] = lo[i];
+          on[8 + i] = hi[i];
+        }
+      }
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const float tv = ok ? v[i] + (bias ? bias[16 * g + i] : 0.0f) : 0.0f;
-        o[i] = relu ? fmaxf(tv, 0.0f) : tv;
+        if (DGRAD) {
+          o[i] = ok && (!mask || on[i] > 0.0f) ? v[i] : 0.0f;
+        } else {
+          const float tv = ok ? v[i] + (bias ? bias[16 * g + i] : 0.0f) : 0.0f;
+          o[i] = relu ? fmaxf(tv, 0.0f) : tv;
+        }
       }
-      if (outf) {
+      if (!DGRAD && outf) {
 #pragma unroll
         for (int i = 0; i < 16; i += 4)
           *reinterpret_cast<float4 *>(outf + m * COUT + 16 * g + i) =
@@ -946,10 +978,10 @@ __global__ void __launch_bounds__(128)
 }
 
 
-template <int CIN, int COUT, int ZT>
+template <int CIN, int COUT, int ZT, bool DGRAD = false>
 cudaError_t launch_direct(const void *x, int B, int D, int H, int W, const void *w,
-                          const float *bias, int relu, void *out, float *outf, int *status,
-                          cudaStream_t s) {
+                          const float *bias, int relu, const void *mask, void *out, float *outf,
+                          int *status, cudaStream_t s) {
   using C = DirectCfg<CIN, COUT, ZT>;
   PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
   if (!encode) return cudaErrorNotSupported;
@@ -965,13 +997,14 @@ cudaError_t launch_direct(const void *x, int B, int D, int H, int W, const void 
              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return cudaErrorNotSupported;
-  auto kern = k_conv_direct<CIN, COUT, ZT>;
+  auto kern = k_conv_direct<CIN, COUT, ZT, DGRAD>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem());
   if (e != cudaSuccess) return e;
   const unsigned grid = (unsigned)((long)B * (D / ZT) * (H / 16) * (W / 8));
   kern<<<grid, 128, C::smem(), s>>>(tmap, static_cast<const bf16 *>(w), bias, relu,
-                                     static_cast<bf16 *>(out), outf, D, H, W, status);
+                                     static_cast<const bf16 *>(mask), static_cast<bf16 *>(out), outf,
+                                     D, H, W, status);
   return cudaGetLastError();
 }
 
@@ -984,14 +1017,9 @@ size_t direct_smem(int zt) {
 // planes per tile for the direct kernel (0: the GEMM path): the deepest tile
 // whose grid still gives two CTAs per SM, else the shallowest (the most
 // CTAs), within two CTAs' shared memory per SM
-int direct_planes(int cin, int cout, int ntaps, int B, int D, int H, int W, int sms) {
+int direct_planes(size_t (*smem)(int), int ntaps, int B, int D, int H, int W, int sms) {
   // the input box (10 x 18 x (planes + 2) voxels) stays within the tensor's extents
   if (ntaps != 27 || W % 8 || H % 16 || W < 16 || H < 32 || B < 1 || D < 3) return 0;
-  size_t (*smem)(int) = nullptr;
-  if (cin == 16 && cout == 16) smem = direct_smem<16, 16>;
-  else if (cin == 48 && cout == 16) smem = direct_smem<48, 16>;
-  else if (cin == 16 && cout == 32) smem = direct_smem<16, 32>;
-  else if (cin == 32 && cout == 32) smem = direct_smem<32, 32>;
   if (!smem) return 0;
   int shallowest = 0;
   for (int zt : {4, 2, 1}) {
@@ -1002,27 +1030,43 @@ int direct_planes(int cin, int cout, int ntaps, int B, int D, int H, int W, int 
   return shallowest;
 }
 
-template <int CIN, int COUT>
-cudaError_t direct_zt(int zt, const void *x, int B, int D, int H, int W, const void *w,
-                      const float *bias, int relu, void *out, float *outf, int *status,
-                      cudaStream_t s) {
-  if (zt == 4) return launch_direct<CIN, COUT, 4>(x, B, D, H, W, w, bias, relu, out, outf, status, s);
-  if (zt == 2) return launch_direct<CIN, COUT, 2>(x, B, D, H, W, w, bias, relu, out, outf, status, s);
-  return launch_direct<CIN, COUT, 1>(x, B, D, H, W, w, bias, relu, out, outf, status, s);
+// f(Cin, Cout) as integral constants for the shapes the direct kernel takes:
+// forward layers, and (dgrad) their data gradients, whose input has the
+// layer's output channels. A shape whose weights leave no room for two CTAs
+// per SM (96 channels) stays on the GEMM.
+template <class F>
+void direct_shape(bool dgrad, int cin, int cout, const F &f) {
+  using std::integral_constant;
+  if (cin == 16 && cout == 16) f(integral_constant<int, 16>(), integral_constant<int, 16>());
+  if (cin == 32 && cout == 32) f(integral_constant<int, 32>(), integral_constant<int, 32>());
+  if (!dgrad && cin == 48 && cout == 16) f(integral_constant<int, 48>(), integral_constant<int, 16>());
+  if (!dgrad && cin == 16 && cout == 32) f(integral_constant<int, 16>(), integral_constant<int, 32>());
+  if (dgrad && cin == 16 && cout == 48) f(integral_constant<int, 16>(), integral_constant<int, 48>());
+  if (dgrad && cin == 32 && cout == 16) f(integral_constant<int, 32>(), integral_constant<int, 16>());
+}
+int direct_planes(bool dgrad, int cin, int cout, int ntaps, int B, int D, int H, int W, int sms) {
+  size_t (*smem)(int) = nullptr;
+  direct_shape(dgrad, cin, cout, [&](auto ci, auto co) {
+    smem = direct_smem<decltype(ci)::value, decltype(co)::value>;
+  });
+  return direct_planes(smem, ntaps, B, D, H, W, sms);
 }
 
+template <bool DGRAD>
 cudaError_t conv_direct(int zt, const void *x, int B, int D, int H, int W, int cin, const void *w,
-                        const float *bias, int cout, int relu, void *out, float *outf,
-                        int *status, cudaStream_t s) {
-  if (cin == 16 && cout == 16)
-    return direct_zt<16, 16>(zt, x, B, D, H, W, w, bias, relu, out, outf, status, s);
-  if (cin == 48 && cout == 16)
-    return direct_zt<48, 16>(zt, x, B, D, H, W, w, bias, relu, out, outf, status, s);
-  if (cin == 16 && cout == 32)
-    return direct_zt<16, 32>(zt, x, B, D, H, W, w, bias, relu, out, outf, status, s);
-  if (cin == 32 && cout == 32)
-    return direct_zt<32, 32>(zt, x, B, D, H, W, w, bias, relu, out, outf, status, s);
-  return cudaErrorInvalidValue;
+                        const float *bias, int cout, int relu, const void *mask, void *out,
+                        float *outf, int *status, cudaStream_t s) {
+  cudaError_t e = cudaErrorInvalidValue;
+  direct_shape(DGRAD, cin, cout, [&](auto ci, auto co) {
+    constexpr int CI = decltype(ci)::value, CO = decltype(co)::value;
+    if (zt == 4)
+      e = launch_direct<CI, CO, 4, DGRAD>(x, B, D, H, W, w, bias, relu, mask, out, outf, status, s);
+    else if (zt == 2)
+      e = launch_direct<CI, CO, 2, DGRAD>(x, B, D, H, W, w, bias, relu, mask, out, outf, status, s);
+    else
+      e = launch_direct<CI, CO, 1, DGRAD>(x, B, D, H, W, w, bias, relu, mask, out, outf, status, s);
+  });
+  return e;
 }
 
 }  // namespace
@@ -1033,12 +1077,16 @@ cudaError_t conv_direct(int zt, const void *x, int B, int D, int H, int W, int c
 static int g_gemm_only = 0;
 void nn_set_gemm_only(int on) { g_gemm_only = on ? 1 : 0; }
 
-int nn_conv_direct_planes(int B, int D, int H, int W, int cin, int cout, int ntaps) {
-  if (g_gemm_only) return 0;
+static int sm_count() {
   int sms = 148, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return direct_planes(cin, cout, ntaps, B, D, H, W, sms);
+  return sms;
+}
+
+int nn_conv_direct_planes(int B, int D, int H, int W, int cin, int cout, int ntaps) {
+  if (g_gemm_only) return 0;
+  return direct_planes(false, cin, cout, ntaps, B, D, H, W, sm_count());
 }
 
 bool nn_channels_ok(int c) { return dispatch_bn(c, [](auto) {}); }
@@ -1113,7 +1161,7 @@ cudaError_t nn_conv_fwd(const void *x, int B, int D, int H, int W, int cin, cons
   if (zt > 0) {
     // cudaErrorNotSupported: no tensor map for this tensor (nothing launched)
     const cudaError_t e =
-        conv_direct(zt, x, B, D, H, W, cin, w, bias, cout, relu, out, outf, status, s);
+        conv_direct<false>(zt, x, B, D, H, W, cin, w, bias, cout, relu, nullptr, out, outf, status, s);
     if (e != cudaErrorNotSupported) return e;
   }
   return conv_gemm<FwdTag>(x, make_vol(B, D, H, W), cin, ntaps, 1, w, cout, M, bias, relu, out,
@@ -1124,6 +1172,12 @@ cudaError_t nn_conv_dgrad(const void *dy, int B, int D, int H, int W, int cout, 
                           int cin, int ntaps, const void *mask, void *dx, float *scratch,
                           size_t scratch_floats, int *status, cudaStream_t s) {
   const long M = (long)B * D * H * W;
+  const int zt = g_gemm_only ? 0 : direct_planes(true, cout, cin, ntaps, B, D, H, W, sm_count());
+  if (zt > 0 && al16(mask)) {
+    const cudaError_t e = conv_direct<true>(zt, dy, B, D, H, W, cout, wt, nullptr, cin, 0, mask, dx,
+                                            nullptr, status, s);
+    if (e != cudaErrorNotSupported) return e;
+  }
   return conv_gemm<DgradTag>(dy, make_vol(B, D, H, W), cout, ntaps, -1, wt, cin, M, nullptr, 0,
                              dx, nullptr, mask, scratch, scratch_floats, status, s);
 }
@@ -1162,7 +1216,7 @@ size_t nn_bias_scratch_floats(long M, int N) {
 cudaError_t nn_bias_grad(const void *dy, long M, int N, float *scratch, float *db, cudaStream_t s) {
   const int nb = (int)((M + kBiasRows - 1) / kBiasRows);
   k_bias_partial<<<nb, kEw, 0, s>>>(static_cast<const bf16 *>(dy), M, N, scratch);
-  k_bias_final<<<1, 256, 0, s>>>(scratch, nb, N, db);
+  k_bias_final<<<N, kEw, 0, s>>>(scratch, nb, N, db);
   return cudaGetLastError();
 }
 
