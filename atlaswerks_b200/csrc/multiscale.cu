@@ -100,24 +100,29 @@ __global__ void __launch_bounds__(kRowThreads)
   v[2 * n + p.i] = fsub(hz[p.i], __int2float_rn(p.z));
 }
 
+// r: coarse voxels per fine voxel along an axis, o: the first fine voxel's
+// place on the coarse grid, scale: the vectors' 1 / r (1 without rescaling)
+struct UpAxis {
+  double r, o;
+  float scale;
+};
+
 __global__ void __launch_bounds__(kRowThreads)
     k_upsample_field(const float *__restrict__ v, Dims din, float *__restrict__ ox,
-                     float *__restrict__ oy, float *__restrict__ oz, Dims dout, int rescale) {
+                     float *__restrict__ oy, float *__restrict__ oz, Dims dout, UpAxis X, UpAxis Y,
+                     UpAxis Z, int rescale) {
   Voxel p;
   if (!voxel_of(dout, p)) return;
-  const double rX = (double)din.nx / dout.nx, rY = (double)din.ny / dout.ny,
-               rZ = (double)din.nz / dout.nz;
-  const double oX = (rX - 1.0) / 2.0, oY = (rY - 1.0) / 2.0, oZ = (rZ - 1.0) / 2.0;
-  const float ix = __double2float_rn(dadd(oX, dmul((double)p.x, rX)));
-  const float iy = __double2float_rn(dadd(oY, dmul((double)p.y, rY)));
-  const float iz = __double2float_rn(dadd(oZ, dmul((double)p.z, rZ)));
+  const float ix = __double2float_rn(dadd(X.o, dmul((double)p.x, X.r)));
+  const float iy = __double2float_rn(dadd(Y.o, dmul((double)p.y, Y.r)));
+  const float iz = __double2float_rn(dadd(Z.o, dmul((double)p.z, Z.r)));
   const long n = din.n();
   float a, b, c;
   trilerp_vector(v, v + n, v + 2 * n, din, ix, iy, iz, BG_CLAMP, 1.0f, a, b, c);
   if (rescale) {
-    a = fmul(a, __double2float_rn(1.0 / rX));
-    b = fmul(b, __double2float_rn(1.0 / rY));
-    c = fmul(c, __double2float_rn(1.0 / rZ));
+    a = fmul(a, X.scale);
+    b = fmul(b, Y.scale);
+    c = fmul(c, Z.scale);
   }
   ox[p.i] = fadd(__int2float_rn(p.x), a);
   oy[p.i] = fadd(__int2float_rn(p.y), b);
@@ -285,8 +290,13 @@ cudaError_t upsample_hfield(const float *const h[3], Dims din, float *const out[
                             int rescale, void *scratch, cudaStream_t s) {
   float *v = static_cast<float *>(scratch);
   k_h_to_v<<<row_grid(din), kRowThreads, 0, s>>>(h[0], h[1], h[2], v, din);
-  k_upsample_field<<<row_grid(dout), kRowThreads, 0, s>>>(v, din, out[0], out[1], out[2], dout,
-                                                          rescale);
+  auto axis = [](int in, int n) {
+    const double r = (double)in / n;
+    return UpAxis{r, (r - 1.0) / 2.0, (float)(1.0 / r)};
+  };
+  k_upsample_field<<<row_grid(dout), kRowThreads, 0, s>>>(
+      v, din, out[0], out[1], out[2], dout, axis(din.nx, dout.nx), axis(din.ny, dout.ny),
+      axis(din.nz, dout.nz), rescale);
   return cudaGetLastError();
 }
 
