@@ -129,6 +129,7 @@ SIGNATURES = {
     "aw_nn_mse_scratch_doubles": ([ctypes.c_long], ctypes.c_size_t),
     "aw_nn_mse": ([_fp, _fp, ctypes.c_long, _fp, _fp, _fp, _fp], _i),
     "aw_nn_adam": ([_fp, _fp, _fp, _fp, ctypes.c_long, _f, _f, _f, _f, _i, _fp], _i),
+    "aw_nn_adam_all": ([_fp, _i, _f, _f, _f, _f, _i, _fp], _i),
     "aw_nn_weights_bf16": ([_fp, _i, _i, _i, _fp, _fp, _fp], _i),
     "aw_nn_displacement_to_h": ([_fp, _i, _i, _i, _fp, _fp, _fp, _fp], _i),
     "aw_nn_status": ([_fp], _i),

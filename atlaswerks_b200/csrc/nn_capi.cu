@@ -36,6 +36,9 @@ cudaError_t nn_mse(const float *pred, const float *tgt, long voxels, void *grad,
                    float *loss, cudaStream_t s);
 cudaError_t nn_adam(float *w, const float *g, float *m1, float *m2, long n, float lr, float b1,
                     float b2, float eps, int t, cudaStream_t s);
+int nn_adam_max();
+cudaError_t nn_adam_all(const aw_nn_adam_item *items, int count, float lr, float b1, float b2, float eps,
+                        int t, cudaStream_t s);
 cudaError_t nn_weights_bf16(const float *w, int cout, int ntaps, int cin, void *wb, void *wt,
                             cudaStream_t s);
 cudaError_t nn_disp_to_h(const float *pred, int D, int H, int W, float *hx, float *hy, float *hz,
@@ -215,6 +218,22 @@ int aw_nn_adam(float *w, const float *g, float *m1, float *m2, long n, float lr,
   return 0;
 }
 
+int aw_nn_adam_all(const aw_nn_adam_item *items, int count, float lr, float beta1, float beta2,
+                   float eps, int step, void *stream) {
+  if (!items) return nfail("aw_nn_adam_all: null pointer");
+  if (count < 1 || count > aw::nn_adam_max()) return nfail("aw_nn_adam_all: 1 to 32 parameters");
+  if (step < 1) return nfail("aw_nn_adam_all: step counts from 1");
+  for (int i = 0; i < count; ++i) {
+    const aw_nn_adam_item &a = items[i];
+    if (!a.w || !a.g || !a.m1 || !a.m2) return nfail("aw_nn_adam_all: null pointer");
+    if (a.n < 1 || a.n >= (1L << 30)) return nfail("aw_nn_adam_all: parameter size");
+    if (a.w_bf16 && (a.cout < 1 || a.ntaps < 1 || a.cin < 1 ||
+                     (long)a.cout * a.ntaps * a.cin != a.n))
+      return nfail("aw_nn_adam_all: weight shape does not match its size");
+  }
+  NN_CUDA(aw::nn_adam_all(items, count, lr, beta1, beta2, eps, step, S(stream)), "aw_nn_adam_all");
+  return 0;
+}
 int aw_nn_weights_bf16(const float *w, int cout, int ntaps, int cin, void *w_bf16,
                        void *wt_bf16, void *stream) {
   if (!w || !w_bf16) return nfail("aw_nn_weights_bf16: null pointer");

@@ -48,6 +48,14 @@ def _p(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
+class _AdamItem(ctypes.Structure):
+    """aw_nn_adam_item"""
+    _fields_ = [("w", ctypes.c_void_p), ("m1", ctypes.c_void_p), ("m2", ctypes.c_void_p),
+                ("g", ctypes.c_void_p), ("w_bf16", ctypes.c_void_p), ("wt_bf16", ctypes.c_void_p),
+                ("n", ctypes.c_long), ("cout", ctypes.c_int), ("ntaps", ctypes.c_int),
+                ("cin", ctypes.c_int)]
+
+
 class WarmStartNet:
     """The network on one grid (D, H, W divisible by 8), batch 1."""
 
@@ -251,14 +259,16 @@ class WarmStartNet:
 
     def adam_step(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8):
         self.t += 1
-        L, s = _lib.lib(), _stream()
-        for name, ci, co, t in LAYERS:
-            check(L.aw_nn_adam(_p(self.w[name]), _p(self.gw[name]), _p(self.m1[name]),
-                               _p(self.m2[name]), self.w[name].numel(), lr, beta1, beta2, eps,
-                               self.t, s))
-            check(L.aw_nn_adam(_p(self.b[name]), _p(self.gb[name]), _p(self.bm1[name]),
-                               _p(self.bm2[name]), co, lr, beta1, beta2, eps, self.t, s))
-        self.refresh_bf16()
+        # every parameter and the weights' BF16 copies in one launch
+        items = (_AdamItem * (2 * len(LAYERS)))()
+        for k, (name, ci, co, t) in enumerate(LAYERS):
+            w = self.w[name]
+            items[2 * k] = _AdamItem(_p(w), _p(self.m1[name]), _p(self.m2[name]), _p(self.gw[name]),
+                                     _p(self.wb[name]), _p(self.wt[name]), w.numel(), co, t, ci)
+            items[2 * k + 1] = _AdamItem(_p(self.b[name]), _p(self.bm1[name]), _p(self.bm2[name]),
+                                         _p(self.gb[name]), None, None, co, 0, 0, 0)
+        check(_lib.lib().aw_nn_adam_all(ctypes.addressof(items), len(items), lr, beta1, beta2, eps,
+                                        self.t, _stream()))
 
     def train_step(self, I0, I1, target, lr=1e-3) -> torch.Tensor:
         self.forward(I0, I1)

@@ -507,6 +507,18 @@ int aw_nn_mse(const float *pred, const float *target, long voxels, void *grad, d
 /* Adam on FP32 masters (step counts from 1) */
 int aw_nn_adam(float *w, const float *g, float *m1, float *m2, long n, float lr, float beta1,
                float beta2, float eps, int step, void *stream);
+/* aw_nn_adam on up to 32 parameters in one launch; a weight tensor
+ * [cout][ntaps][cin] with w_bf16 set also gets its BF16 copies, as
+ * aw_nn_weights_bf16 writes them (wt_bf16 may be null). */
+typedef struct {
+  float *w, *m1, *m2;
+  const float *g;
+  void *w_bf16, *wt_bf16;
+  long n;
+  int cout, ntaps, cin;
+} aw_nn_adam_item;
+int aw_nn_adam_all(const aw_nn_adam_item *items, int count, float lr, float beta1, float beta2,
+                   float eps, int step, void *stream);
 /* BF16 copies of FP32 weights: [Cout][taps][Cin] and (wt_bf16 non-NULL)
  * the transposed [Cin][taps][Cout] */
 int aw_nn_weights_bf16(const float *w, int cout, int ntaps, int cin, void *w_bf16,
