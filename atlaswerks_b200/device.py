@@ -41,6 +41,14 @@ def _p(t: torch.Tensor) -> int:
     return t.data_ptr()
 
 
+def _planes(t: torch.Tensor):
+    """The addresses of a contiguous field's three planes (one tensor call
+    instead of an indexed view each)."""
+    p = t.data_ptr()
+    n = t.numel() // t.shape[0] * t.element_size()
+    return p, p + n, p + 2 * n
+
+
 def identity(shape: Sequence[int], device="cuda") -> torch.Tensor:
     nz, ny, nx = shape
     z, y, x = torch.meshgrid(torch.arange(nz, device=device), torch.arange(ny, device=device),

@@ -28,7 +28,7 @@ import torch
 
 from . import _lib
 from ._lib import check
-from .device import _check_field, _check_image, _dims, _stream, identity
+from .device import _check_field, _check_image, _dims, _planes, _stream, identity
 
 
 @dataclass
@@ -70,8 +70,7 @@ class DiffOperB200:
             raise RuntimeError("SetSize() must be called first")
         if tuple(v.shape[1:]) != (self.size[2], self.size[1], self.size[0]):
             raise ValueError("field size does not match SetSize()")
-        check(_lib.lib().aw_fluid_apply(self._h, v[0].data_ptr(), v[1].data_ptr(),
-                                        v[2].data_ptr(), inverse, _stream()))
+        check(_lib.lib().aw_fluid_apply(self._h, *_planes(v), inverse, _stream()))
         return v
 
     def ApplyOperator(self, v: torch.Tensor) -> torch.Tensor:
@@ -143,8 +142,7 @@ class GreedyDeformationDataB200:
         self._cur = 0
         nx, ny, nz = _dims(self.I0)
         for h in [self._h[0]] + ([self._hi[0]] if self._hi else []):
-            check(_lib.lib().aw_identity(h[0].data_ptr(), h[1].data_ptr(), h[2].data_ptr(),
-                                         nx, ny, nz, _stream()))
+            check(_lib.lib().aw_identity(*_planes(h), nx, ny, nz, _stream()))
 
     def Def1To0(self) -> torch.Tensor:
         return self._h[self._cur]
@@ -211,10 +209,9 @@ class GreedyIteratorB200:
         h, hi = data.Def1To0(), (data.Def0To1() if data.ComputeInverseHField() else None)
         ho, hio = data._next()
         z = [None, None, None]
-        hp = [t.data_ptr() for t in h]
-        op = [t.data_ptr() for t in ho]
-        hip = [t.data_ptr() for t in hi] if hi is not None else z
-        iop = [t.data_ptr() for t in hio] if hio is not None else z
+        hp, op = _planes(h), _planes(ho)
+        hip = _planes(hi) if hi is not None else z
+        iop = _planes(hio) if hio is not None else z
         check(_lib.lib().aw_greedy_iterate(self._h, data.I0.data_ptr(), data.I1.data_ptr(), *hp,
                                            *op, *hip, *iop, int(self._update_step), _stream()))
         self._update_step = False
@@ -226,12 +223,12 @@ class GreedyIteratorB200:
         z = [None, None, None]
         if data.ComputeInverseHField():
             hi, si = data.Def0To1(), data._next()[1]
-            hip, sip = [t.data_ptr() for t in hi], [t.data_ptr() for t in si]
+            hip, sip = _planes(hi), _planes(si)
         else:
             hip, sip = z, z
         check(_lib.lib().aw_greedy_run(self._h, data.I0.data_ptr(), data.I1.data_ptr(),
-                                       *[t.data_ptr() for t in h], *[t.data_ptr() for t in s],
-                                       *hip, *sip, int(n_iters), int(update_first), _stream()))
+                                       *_planes(h), *_planes(s), *hip, *sip, int(n_iters),
+                                       int(update_first), _stream()))
 
     def Energies(self) -> np.ndarray:
         n = ctypes.c_int()
