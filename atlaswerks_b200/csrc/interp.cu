@@ -18,6 +18,7 @@ constexpr int kThreads = kRowThreads;
 __global__ void __launch_bounds__(kThreads)
     k_apply(const float *__restrict__ img, const float *__restrict__ hx, const float *__restrict__ hy,
             const float *__restrict__ hz, float *__restrict__ out, Dims d, float bg) {
+  early_entry();
   Voxel vx;
   if (!voxel_of(d, vx)) return;
   const long i = vx.i;
@@ -32,6 +33,7 @@ struct AxisDiv {
 __global__ void __launch_bounds__(kThreads)
     k_gradient(const float *__restrict__ a, float *__restrict__ gx, float *__restrict__ gy,
                float *__restrict__ gz, Dims d, AxisDiv c2, AxisDiv c1, int wrap) {
+  early_entry();
   Voxel vx;
   if (!voxel_of(d, vx)) return;
   const long i = vx.i;
@@ -65,6 +67,7 @@ __global__ void __launch_bounds__(kThreads)
                  float *__restrict__ ox, float *__restrict__ oy, float *__restrict__ oz, Dims d,
                  DivF q0, DivF q1, DivF q2, int dir, int bgs, const float *__restrict__ scale_ptr,
                  float scale_val) {
+  early_entry();
   Voxel vox;
   if (!voxel_of(d, vox)) return;
   const long i = vox.i;
@@ -94,6 +97,7 @@ __global__ void __launch_bounds__(kThreads)
                  float *__restrict__ ox, float *__restrict__ oy, float *__restrict__ oz, Dims d,
                  DivF q0, DivF q1, DivF q2, int dir, int bgs, const float *__restrict__ scale_ptr,
                  float scale_val) {
+  early_entry();
   Voxel vox;
   if (!voxel_of(d, vox)) return;
   const long i = vox.i;
@@ -114,7 +118,7 @@ __global__ void __launch_bounds__(kThreads)
 
 cudaError_t launch_apply(const float *img, const float *hx, const float *hy, const float *hz,
                          float *out, Dims d, float bg, cudaStream_t s) {
-  k_apply<<<row_grid(d), kThreads, 0, s>>>(img, hx, hy, hz, out, d, bg);
+  launch_early(k_apply, row_grid(d), kThreads, 0, s, img, hx, hy, hz, out, d, bg);
   return cudaGetLastError();
 }
 
@@ -122,27 +126,25 @@ cudaError_t launch_gradient(const float *a, float *gx, float *gy, float *gz, Dim
                             int wrap, cudaStream_t s) {
   const AxisDiv c2{{make_div(2.0 * sp.x), make_div(2.0 * sp.y), make_div(2.0 * sp.z)}};
   const AxisDiv c1{{make_div(sp.x), make_div(sp.y), make_div(sp.z)}};
-  k_gradient<<<row_grid(d), kThreads, 0, s>>>(a, gx, gy, gz, d, c2, c1, wrap);
+  launch_early(k_gradient, row_grid(d), kThreads, 0, s, a, gx, gy, gz, d, c2, c1, wrap);
   return cudaGetLastError();
 }
 
 cudaError_t launch_compose_hv(const float *const g[3], const float *const v[3], float *const o[3],
                               Dims d, Spacing sp, int dir, int bgs, const float *scale_ptr,
                               float scale_val, cudaStream_t s) {
-  k_compose_hv<<<row_grid(d), kThreads, 0, s>>>(g[0], g[1], g[2], v[0], v[1], v[2], o[0], o[1],
-                                                    o[2], d, make_divf((float)sp.x), make_divf((float)sp.y),
-                                                    make_divf((float)sp.z), dir, bgs, scale_ptr,
-                                                    scale_val);
+  launch_early(k_compose_hv, row_grid(d), kThreads, 0, s, g[0], g[1], g[2], v[0], v[1], v[2], o[0],
+               o[1], o[2], d, make_divf((float)sp.x), make_divf((float)sp.y),
+               make_divf((float)sp.z), dir, bgs, scale_ptr, scale_val);
   return cudaGetLastError();
 }
 
 cudaError_t launch_compose_vh(const float *const v[3], const float *const g[3], float *const o[3],
                               Dims d, Spacing sp, int dir, int bgs, const float *scale_ptr,
                               float scale_val, cudaStream_t s) {
-  k_compose_vh<<<row_grid(d), kThreads, 0, s>>>(v[0], v[1], v[2], g[0], g[1], g[2], o[0], o[1],
-                                                    o[2], d, make_divf((float)sp.x), make_divf((float)sp.y),
-                                                    make_divf((float)sp.z), dir, bgs, scale_ptr,
-                                                    scale_val);
+  launch_early(k_compose_vh, row_grid(d), kThreads, 0, s, v[0], v[1], v[2], g[0], g[1], g[2], o[0],
+               o[1], o[2], d, make_divf((float)sp.x), make_divf((float)sp.y),
+               make_divf((float)sp.z), dir, bgs, scale_ptr, scale_val);
   return cudaGetLastError();
 }
 

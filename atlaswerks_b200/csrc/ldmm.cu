@@ -27,6 +27,7 @@ namespace {
 
 __global__ void __launch_bounds__(kRowThreads)
     k_identity(float *__restrict__ hx, float *__restrict__ hy, float *__restrict__ hz, Dims d) {
+  early_entry();
   Voxel v;
   if (!voxel_of(d, v)) return;
   hx[v.i] = __int2float_rn(v.x);
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(kRowThreads)
                    const float *__restrict__ vy, const float *__restrict__ vz,
                    float *__restrict__ ox, float *__restrict__ oy, float *__restrict__ oz,
                    const float *__restrict__ I0, float *__restrict__ J, Dims d, SpaceDiv sp) {
+  early_entry();
   Voxel vox;
   if (!voxel_of(d, vox)) return;
   const long i = vox.i;
@@ -101,6 +103,7 @@ __global__ void __launch_bounds__(kRowThreads)
              const float *__restrict__ vz, const float *__restrict__ next,
              float *__restrict__ out, Dims d, SpaceDiv sp, DivD a2, DivD b2, DivD e2, DivD a1,
              DivD b1, DivD e1) {
+  early_entry();
   Voxel vox;
   if (!voxel_of(d, vox)) return;
   const int x = vox.x, y = vox.y, z = vox.z;
@@ -131,6 +134,7 @@ __global__ void __launch_bounds__(kRowThreads)
 __global__ void __launch_bounds__(kRowThreads)
     k_residual(const float *__restrict__ J, const float *__restrict__ I1, float *__restrict__ diff,
                double *__restrict__ partials, Dims d) {
+  early_entry();
   Voxel v;
   double e = 0.0;
   if (voxel_of(d, v)) {
@@ -159,6 +163,7 @@ __global__ void __launch_bounds__(kRecThreads)
     k_record_energy(const double *__restrict__ partials, int nparts, double scale,
                     double *__restrict__ energy, int *__restrict__ count, int cap,
                     int advance = 1, int add = 0, int back = 0) {
+  early_entry();
   double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
   int i = threadIdx.x;
   for (; i + 3 * kRecThreads < nparts; i += 4 * kRecThreads) {
@@ -189,6 +194,7 @@ __global__ void __launch_bounds__(256)
                const float *__restrict__ vz, const float *__restrict__ ux,
                const float *__restrict__ uy, const float *__restrict__ uz, long n, float sigma,
                unsigned *__restrict__ maxbits) {
+  early_entry();
   const float a = 2.0f, b = fdiv(-2.0f, fmul(sigma, sigma));
   float m = 0.0f;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
@@ -203,6 +209,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void k_step_from_max(const unsigned *__restrict__ maxbits, float max_pert,
                                 float *__restrict__ step) {
+  early_entry();
   *step = fdiv(max_pert, __uint_as_float(*maxbits));
 }
 
@@ -247,6 +254,7 @@ __global__ void __launch_bounds__(kRowThreads)
     k_ad_force(const float *__restrict__ aHat, const float *__restrict__ aT,
                const float *__restrict__ IT, const float *__restrict__ IHat, float *__restrict__ fx,
                float *__restrict__ fy, float *__restrict__ fz, Dims d, GradDiv g) {
+  early_entry();
   Voxel v;
   if (!voxel_of(d, v)) return;
   const float at = __ldg(aT + v.i), ih = __ldg(IHat + v.i);
@@ -265,6 +273,7 @@ __global__ void __launch_bounds__(kRowThreads)
                  const float *__restrict__ vy, const float *__restrict__ vz,
                  const float *__restrict__ aT, float *__restrict__ dot, float *__restrict__ div,
                  Dims d, GradDiv g) {
+  early_entry();
   Voxel v;
   if (!voxel_of(d, v)) return;
   const float *const vc[3] = {vx, vy, vz};
@@ -290,6 +299,7 @@ __global__ void __launch_bounds__(kRowThreads)
     k_ad_pull(const float *__restrict__ src, const float *__restrict__ hx,
               const float *__restrict__ hy, const float *__restrict__ hz, float *__restrict__ out,
               Dims d) {
+  early_entry();
   Voxel v;
   if (!voxel_of(d, v)) return;
   const float r = trilerp_scalar(src, d, __ldg(hx + v.i), __ldg(hy + v.i), __ldg(hz + v.i), 0.0f);
@@ -298,6 +308,7 @@ __global__ void __launch_bounds__(kRowThreads)
 
 __global__ void __launch_bounds__(256) k_ad_add(float *__restrict__ a, const float *__restrict__ b,
                                                 long n) {
+  early_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] = fadd(a[i], b[i]);
 }
@@ -307,6 +318,7 @@ __global__ void __launch_bounds__(256) k_ad_add(float *__restrict__ a, const flo
 __global__ void __launch_bounds__(kRowThreads)
     k_ad_residual(const float *__restrict__ J, const float *__restrict__ I1, float inv,
                   float *__restrict__ ihat, double *__restrict__ partials, Dims d) {
+  early_entry();
   Voxel v;
   double e = 0.0;
   if (voxel_of(d, v)) {
@@ -336,6 +348,7 @@ __global__ void __launch_bounds__(kRowThreads)
 __global__ void __launch_bounds__(kRowThreads)
     k_force_vdot(SrcForce f, const float *__restrict__ v, float sign,
                  double *__restrict__ partials, Dims d) {
+  early_entry();
   Voxel p;
   double e = 0.0;
   if (voxel_of(d, p)) {
@@ -361,6 +374,7 @@ __global__ void __launch_bounds__(kRowThreads)
 __global__ void __launch_bounds__(kRowThreads)
     k_field_dot(const float *__restrict__ u, const float *__restrict__ v,
                 double *__restrict__ partials, Dims d) {
+  early_entry();
   Voxel p;
   double e = 0.0;
   if (voxel_of(d, p)) {
@@ -386,6 +400,7 @@ __global__ void __launch_bounds__(kRowThreads)
     k_ad_alpha(const float *__restrict__ I0, const float *__restrict__ v0,
                const float *__restrict__ aTil, const float *__restrict__ step,
                float *__restrict__ alpha0, Dims d, GradDiv g) {
+  early_entry();
   Voxel v;
   if (!voxel_of(d, v)) return;
   const long n = d.n();
@@ -458,7 +473,7 @@ cudaError_t ldmm_iterate_orig(LdmmCtx *c, const float *I0, const float *I1, floa
                               int update_step, cudaStream_t s);
 
 cudaError_t identity_field(float *hx, float *hy, float *hz, Dims d, cudaStream_t s) {
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(hx, hy, hz, d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, hx, hy, hz, d);
   return cudaGetLastError();
 }
 
@@ -475,19 +490,20 @@ cudaError_t ldmm_forward(LdmmCtx *c, const float *I0, const float *I1, const flo
   float *H[2] = {c->hbuf, c->hbuf + 3 * n};
   auto comp = [&](float *base, int k) { return base + k * n; };
   auto vcomp = [&](const float *base, int k) { return base + k * n; };
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(comp(H[0], 0), comp(H[0], 1), comp(H[0], 2), d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, comp(H[0], 0), comp(H[0], 1),
+               comp(H[0], 2), d);
   AW_TRY(cudaGetLastError());
   int cur = 0;
   for (int i = 0; i < T; ++i) {
     const float *vi = v + (long)i * 3 * n;
-    k_forward_step<false><<<row_grid(d), kRowThreads, 0, s>>>(
-        comp(H[cur], 0), comp(H[cur], 1), comp(H[cur], 2), vcomp(vi, 0), vcomp(vi, 1),
-        vcomp(vi, 2), comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I0,
-        c->J0 + (long)i * n, d, space_div(c->sp));
+    launch_early(k_forward_step<false>, row_grid(d), kRowThreads, 0, s, comp(H[cur], 0),
+                 comp(H[cur], 1), comp(H[cur], 2), vcomp(vi, 0), vcomp(vi, 1), vcomp(vi, 2),
+                 comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I0,
+                 c->J0 + (long)i * n, d, space_div(c->sp));
     AW_TRY(cudaGetLastError());
     cur = 1 - cur;
   }
-  k_residual<<<row_grid(d), kRowThreads, 0, s>>>(c->J0 + (long)(T - 1) * n, I1, c->diff,
+  launch_early(k_residual, row_grid(d), kRowThreads, 0, s, c->J0 + (long)(T - 1) * n, I1, c->diff,
                                                  c->partials, d);
   AW_TRY(cudaGetLastError());
   if (!update_step) {
@@ -510,7 +526,7 @@ static cudaError_t vec_step_energy(LdmmCtx *c, const float *vt, int t, int first
   AW_TRY(fluid_forward_field(c->plan, vt, vt + n, vt + 2 * n, s));
   AW_TRY(fluid_solve(c->plan, 0, s));
   AW_TRY(fluid_inverse_store(c->plan, u, u + n, u + 2 * n, s));
-  k_field_dot<<<row_grid(c->d), kRowThreads, 0, s>>>(u, vt, c->partials, c->d);
+  launch_early(k_field_dot, row_grid(c->d), kRowThreads, 0, s, u, vt, c->partials, c->d);
   AW_TRY(cudaGetLastError());
   const double spprod = c->sp.x * c->sp.y * c->sp.z;
   k_record_energy<<<1, kRecThreads, 0, s>>>(c->partials, c->nparts, spprod, c->venergy, c->count,
@@ -525,6 +541,7 @@ static cudaError_t vec_step_energy(LdmmCtx *c, const float *vt, int t, int first
 // as Array3D::scale receives it (LDMMIteratorCPU.cxx:583-585)
 __global__ void __launch_bounds__(256)
     k_scale_to(float *__restrict__ dst, const float *__restrict__ src, float f, long n) {
+  early_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = fmul(src[i], f);
 }
@@ -542,7 +559,8 @@ cudaError_t ldmm_alphas(LdmmCtx *c, const float *I0, const float *I1, const floa
   AW_TRY(ldmm_forward(c, I0, I1, v, 0, s));
   float *H[2] = {c->hbuf, c->hbuf + 3 * n};
   auto comp = [&](float *base, int k) { return base + k * n; };
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(comp(H[0], 0), comp(H[0], 1), comp(H[0], 2), d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, comp(H[0], 0), comp(H[0], 1),
+               comp(H[0], 2), d);
   AW_TRY(cudaGetLastError());
   const float f = (float)(1.0 / (double)(c->sigma * c->sigma));
   int cur = 0;
@@ -554,7 +572,8 @@ cudaError_t ldmm_alphas(LdmmCtx *c, const float *I0, const float *I1, const floa
     AW_TRY(launch_compose_vh(vv, hh, oo, d, c->sp, -1, BG_PARTIAL_ZERO, nullptr, 1.0f, s));
     cur = 1 - cur;
     AW_TRY(splat(c->sw, c->diff, comp(H[cur], 0), comp(H[cur], 1), comp(H[cur], 2), c->S, 0.0f, s));
-    k_scale_to<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(alphas + (long)t * n, c->S, f, n);
+    launch_early(k_scale_to, dim3((unsigned)((n + 255) / 256)), 256, 0, s, alphas + (long)t * n,
+                 c->S, f, n);
     AW_TRY(cudaGetLastError());
   }
   return cudaSuccess;
@@ -572,7 +591,8 @@ cudaError_t ldmm_iterate(LdmmCtx *c, const float *I0, const float *I1, float *v,
   if (update_step) AW_TRY(cudaMemsetAsync(c->maxbits, 0, sizeof(unsigned), s));
   int cur = 0;
   // backward sweep
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(comp(H[0], 0), comp(H[0], 1), comp(H[0], 2), d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, comp(H[0], 0), comp(H[0], 1),
+               comp(H[0], 2), d);
   AW_TRY(cudaGetLastError());
   cur = 0;
   for (int t = T - 1; t >= 0; --t) {
@@ -590,8 +610,8 @@ cudaError_t ldmm_iterate(LdmmCtx *c, const float *I0, const float *I1, float *v,
       AW_TRY(fluid_inverse_store(c->plan, comp(c->u, 0), comp(c->u, 1), comp(c->u, 2), s));
       int sms = 148;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->plan.device);
-      k_max_disp<<<sms * 4, 256, 0, s>>>(comp(vt, 0), comp(vt, 1), comp(vt, 2), comp(c->u, 0),
-                                         comp(c->u, 1), comp(c->u, 2), n, c->sigma, c->maxbits);
+      launch_early(k_max_disp, dim3(sms * 4), 256, 0, s, comp(vt, 0), comp(vt, 1), comp(vt, 2),
+                   comp(c->u, 0), comp(c->u, 1), comp(c->u, 2), n, c->sigma, c->maxbits);
       AW_TRY(cudaGetLastError());
     } else {
       AW_TRY(fluid_inverse_axpby(c->plan, comp(vt, 0), comp(vt, 1), comp(vt, 2), c->step,
@@ -601,7 +621,7 @@ cudaError_t ldmm_iterate(LdmmCtx *c, const float *I0, const float *I1, float *v,
     }
   }
   if (update_step) {
-    k_step_from_max<<<1, 1, 0, s>>>(c->maxbits, c->max_pert, c->step);
+    launch_early(k_step_from_max, dim3(1), 1, 0, s, c->maxbits, c->max_pert, c->step);
     AW_TRY(cudaGetLastError());
   }
   return cudaSuccess;
@@ -624,21 +644,22 @@ cudaError_t ldmm_i1_at_0(LdmmCtx *c, const float *I1, const float *v, float *img
   const DivD a2 = make_div(2.0 * c->sp.x), b2 = make_div(2.0 * c->sp.y), e2 = make_div(2.0 * c->sp.z);
   const DivD a1 = make_div(c->sp.x), b1 = make_div(c->sp.y), e1 = make_div(c->sp.z);
   auto jbuf = [&](int t) { return (t % 2 == 0) ? jd : c->S; };
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(comp(H[0], 0), comp(H[0], 1), comp(H[0], 2), d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, comp(H[0], 0), comp(H[0], 1),
+               comp(H[0], 2), d);
   AW_TRY(cudaGetLastError());
   int cur = 0;
   for (int t = T - 1; t >= 0; --t) {
     const float *vt = v + (long)t * 3 * n;
-    k_forward_step<true><<<row_grid(d), kRowThreads, 0, s>>>(
-        comp(H[cur], 0), comp(H[cur], 1), comp(H[cur], 2), vcomp(vt, 0), vcomp(vt, 1),
-        vcomp(vt, 2), comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I1,
-        t == 0 ? img : nullptr, d, space_div(c->sp));
+    launch_early(k_forward_step<true>, row_grid(d), kRowThreads, 0, s, comp(H[cur], 0),
+                 comp(H[cur], 1), comp(H[cur], 2), vcomp(vt, 0), vcomp(vt, 1), vcomp(vt, 2),
+                 comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I1,
+                 t == 0 ? img : nullptr, d, space_div(c->sp));
     AW_TRY(cudaGetLastError());
     cur = 1 - cur;
     if (jd) {
-      k_jacdet<<<row_grid(d), kRowThreads, 0, s>>>(vcomp(vt, 0), vcomp(vt, 1), vcomp(vt, 2),
-                                                   t == T - 1 ? nullptr : jbuf(t + 1), jbuf(t),
-                                                   d, space_div(c->sp), a2, b2, e2, a1, b1, e1);
+      launch_early(k_jacdet, row_grid(d), kRowThreads, 0, s, vcomp(vt, 0), vcomp(vt, 1),
+                   vcomp(vt, 2), t == T - 1 ? nullptr : jbuf(t + 1), jbuf(t), d, space_div(c->sp),
+                   a2, b2, e2, a1, b1, e1);
       AW_TRY(cudaGetLastError());
     }
   }
@@ -652,6 +673,7 @@ namespace {
 __global__ void k_atlas_accumulate(float *__restrict__ acc, float *__restrict__ jsum,
                                    const float *__restrict__ img, const float *__restrict__ jd,
                                    float w, long n) {
+  early_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   if (jd) {
@@ -663,6 +685,7 @@ __global__ void k_atlas_accumulate(float *__restrict__ acc, float *__restrict__ 
 }
 // mean = acc / jsum (RealImage::pointwiseDivideBy, LDMMAtlasBuilder.txx:332-334)
 __global__ void k_atlas_normalize(float *__restrict__ acc, const float *__restrict__ jsum, long n) {
+  early_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) acc[i] = fdiv(acc[i], jsum[i]);
 }
@@ -670,12 +693,13 @@ __global__ void k_atlas_normalize(float *__restrict__ acc, const float *__restri
 
 cudaError_t ldmm_atlas_accumulate(float *acc, float *jsum, const float *img, const float *jd,
                                   float w, long n, cudaStream_t s) {
-  k_atlas_accumulate<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(acc, jsum, img, jd, w, n);
+  launch_early(k_atlas_accumulate, dim3((unsigned)((n + 255) / 256)), 256, 0, s, acc, jsum, img, jd,
+               w, n);
   return cudaGetLastError();
 }
 
 cudaError_t ldmm_atlas_normalize(float *acc, const float *jsum, long n, cudaStream_t s) {
-  k_atlas_normalize<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(acc, jsum, n);
+  launch_early(k_atlas_normalize, dim3((unsigned)((n + 255) / 256)), 256, 0, s, acc, jsum, n);
   return cudaGetLastError();
 }
 
@@ -715,6 +739,7 @@ __device__ __forceinline__ void voxel_min_max(const VoxelImages &in, int nimg, l
 // range[0] / range[1]: order keys of the volume's smallest min and largest max
 __global__ void k_median_range(const __grid_constant__ VoxelImages in, int nimg, long n,
                                unsigned *range) {
+  early_entry();
   __shared__ unsigned lo_s[8], hi_s[8];
   unsigned lo = 0xffffffffu, hi = 0u;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -746,6 +771,7 @@ __global__ void k_median_range(const __grid_constant__ VoxelImages in, int nimg,
 
 __global__ void k_median_select(const __grid_constant__ VoxelImages in, int nimg, unsigned k,
                                 long n, const unsigned *range, float *out, int *open) {
+  early_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float eps = fdiv(fsub(key_value(range[1]), key_value(range[0])), 10000.f);
@@ -803,9 +829,9 @@ cudaError_t ldmm_voxel_median(const VoxelImages &in, int nimg, int k, long n, fl
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long blocks = std::min<long>((n + 255) / 256, 4L * sms);
-  k_median_range<<<(unsigned)blocks, 256, 0, s>>>(in, nimg, n, range);
-  k_median_select<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(in, nimg, (unsigned)k, n, range,
-                                                             out, open);
+  launch_early(k_median_range, dim3((unsigned)blocks), 256, 0, s, in, nimg, n, range);
+  launch_early(k_median_select, dim3((unsigned)((n + 255) / 256)), 256, 0, s, in, nimg, (unsigned)k,
+               n, range, out, open);
   return cudaGetLastError();
 }
 
@@ -815,6 +841,7 @@ namespace {
 // (LDMMShootingIteratorCPU.cxx:287-297)
 __global__ void k_shoot_alpha(float *__restrict__ a0, const float *__restrict__ aT,
                               const float *__restrict__ step, float sigma, long n) {
+  early_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float eps = *step;
@@ -854,7 +881,7 @@ static cudaError_t shoot_geodesic(LdmmCtx *c, const float *I0, const float *alph
     AW_TRY(fluid_solve(c->plan, 1, s));
     AW_TRY(fluid_inverse_store(c->plan, comp(v, 0), comp(v, 1), comp(v, 2), s));
     if (!record) return cudaSuccess;
-    k_force_vdot<<<row_grid(d), kRowThreads, 0, s>>>(make_force(G, aT, 0, c->sp), v, 1.0f,
+    launch_early(k_force_vdot, row_grid(d), kRowThreads, 0, s, make_force(G, aT, 0, c->sp), v, 1.0f,
                                                       c->partials, d);
     AW_TRY(cudaGetLastError());
     k_record_energy<<<1, kRecThreads, 0, s>>>(c->partials, c->nparts, spprod, c->venergy,
@@ -870,15 +897,18 @@ static cudaError_t shoot_geodesic(LdmmCtx *c, const float *I0, const float *alph
     return cudaSuccess;
   };
   auto advance_phiT0 = [&]() -> cudaError_t {  // phiT0 = composeHVInv(phiT0, v), I = I0(phiT0)
-    k_forward_step<false><<<row_grid(d), kRowThreads, 0, s>>>(
-        comp(B[cb], 0), comp(B[cb], 1), comp(B[cb], 2), comp(v, 0), comp(v, 1), comp(v, 2),
-        comp(B[1 - cb], 0), comp(B[1 - cb], 1), comp(B[1 - cb], 2), I0, I, d, space_div(c->sp));
+    launch_early(k_forward_step<false>, row_grid(d), kRowThreads, 0, s, comp(B[cb], 0),
+                 comp(B[cb], 1), comp(B[cb], 2), comp(v, 0), comp(v, 1), comp(v, 2),
+                 comp(B[1 - cb], 0), comp(B[1 - cb], 1), comp(B[1 - cb], 2), I0, I, d,
+                 space_div(c->sp));
     cb = 1 - cb;
     return cudaGetLastError();
   };
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(comp(phi0T, 0), comp(phi0T, 1), comp(phi0T, 2), d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, comp(phi0T, 0), comp(phi0T, 1),
+               comp(phi0T, 2), d);
   AW_TRY(cudaGetLastError());
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(comp(phiT0, 0), comp(phiT0, 1), comp(phiT0, 2), d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, comp(phiT0, 0), comp(phiT0, 1),
+               comp(phiT0, 2), d);
   AW_TRY(cudaGetLastError());
   AW_TRY(cudaMemcpyAsync(aT, alpha0, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
   AW_TRY(velocity(I0));
@@ -906,10 +936,11 @@ cudaError_t ldmm_shoot_iterate(LdmmCtx *c, const float *I0, const float *I1, flo
   AW_TRY(shoot_geodesic(c, I0, alpha0, phi0T, phiT0, true, A, B, ca, cb, s));
   float *aT = c->S, *I = c->J0;
   const double spprod = c->sp.x * c->sp.y * c->sp.z;
-  k_residual<<<row_grid(d), kRowThreads, 0, s>>>(I, I1, c->diff, c->partials, d);
+  launch_early(k_residual, row_grid(d), kRowThreads, 0, s, I, I1, c->diff, c->partials, d);
   AW_TRY(cudaGetLastError());
   AW_TRY(splat(c->sw, c->diff, comp(B[cb], 0), comp(B[cb], 1), comp(B[cb], 2), aT, 0.0f, s));
-  k_shoot_alpha<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(alpha0, aT, c->step, c->sigma, n);
+  launch_early(k_shoot_alpha, dim3((unsigned)((n + 255) / 256)), 256, 0, s, alpha0, aT, c->step,
+               c->sigma, n);
   AW_TRY(cudaGetLastError());
   k_record_energy<<<1, kRecThreads, 0, s>>>(c->partials, c->nparts, spprod, c->energy,
                                             c->count, c->cap);
@@ -938,6 +969,7 @@ namespace {
 
 // D phiT0 = identity: rows x | y | z, each a vector field [3][N]
 __global__ void k_dphi_identity(float *__restrict__ dp, long n) {
+  early_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
 #pragma unroll
@@ -948,6 +980,7 @@ __global__ void k_dphi_identity(float *__restrict__ dp, long n) {
 
 // row += g (Array3D<Vector3D<Real>>::pointwiseAdd), 3N floats
 __global__ void k_add3(float *__restrict__ row, const float *__restrict__ g, long n3) {
+  early_entry();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n3) row[i] = fadd(row[i], g[i]);
 }
@@ -960,6 +993,7 @@ __global__ void __launch_bounds__(kRowThreads)
     k_velshoot_force(const float *__restrict__ dp, const float *__restrict__ lv0,
                      const float *__restrict__ hx, const float *__restrict__ hy,
                      const float *__restrict__ hz, float *__restrict__ f, Dims d) {
+  early_entry();
   Voxel v;
   if (!voxel_of(d, v)) return;
   const long n = d.n(), i = v.i;
@@ -1016,7 +1050,7 @@ cudaError_t ldmm_velshoot_iterate(LdmmCtx *c, const float *I0, const float *I1, 
   const double spprod = c->sp.x * c->sp.y * c->sp.z;
   const unsigned flat = (unsigned)((n + 255) / 256), flat3 = (unsigned)((3 * n + 255) / 256);
   auto record_vec = [&](const float *a, const float *b, int t) -> cudaError_t {
-    k_field_dot<<<row_grid(d), kRowThreads, 0, s>>>(a, b, c->partials, d);
+    launch_early(k_field_dot, row_grid(d), kRowThreads, 0, s, a, b, c->partials, d);
     AW_TRY(cudaGetLastError());
     k_record_energy<<<1, kRecThreads, 0, s>>>(c->partials, c->nparts, spprod, c->venergy,
                                               c->count, c->cap, 0, t > 0 ? 1 : 0, 0);
@@ -1025,12 +1059,14 @@ cudaError_t ldmm_velshoot_iterate(LdmmCtx *c, const float *I0, const float *I1, 
                                               c->zero, 1, 0, 0, 0);
     return cudaGetLastError();
   };
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(comp(phi0T, 0), comp(phi0T, 1), comp(phi0T, 2), d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, comp(phi0T, 0), comp(phi0T, 1),
+               comp(phi0T, 2), d);
   AW_TRY(cudaGetLastError());
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(comp(phiT0, 0), comp(phiT0, 1), comp(phiT0, 2), d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, comp(phiT0, 0), comp(phiT0, 1),
+               comp(phiT0, 2), d);
   AW_TRY(cudaGetLastError());
   AW_TRY(cudaMemcpyAsync(vt, v0, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, s));
-  k_dphi_identity<<<flat, 256, 0, s>>>(dp, n);
+  launch_early(k_dphi_identity, dim3(flat), 256, 0, s, dp, n);
   AW_TRY(cudaGetLastError());
   AW_TRY(fluid_forward_field(c->plan, comp(v0, 0), comp(v0, 1), comp(v0, 2), s));
   AW_TRY(fluid_solve(c->plan, 0, s));
@@ -1056,11 +1092,11 @@ cudaError_t ldmm_velshoot_iterate(LdmmCtx *c, const float *I0, const float *I1, 
       AW_TRY(launch_apply(comp(vt, r), comp(B[cb], 0), comp(B[cb], 1), comp(B[cb], 2), img, d,
                           0.0f, s));
       AW_TRY(launch_gradient(img, comp(g, 0), comp(g, 1), comp(g, 2), d, c->sp, 0, s));
-      k_add3<<<flat3, 256, 0, s>>>(dp + (long)3 * r * n, g, 3 * n);
+      launch_early(k_add3, dim3(flat3), 256, 0, s, dp + (long)3 * r * n, g, 3 * n);
       AW_TRY(cudaGetLastError());
     }
-    k_velshoot_force<<<row_grid(d), kRowThreads, 0, s>>>(dp, lv0, comp(B[cb], 0), comp(B[cb], 1),
-                                                         comp(B[cb], 2), f, d);
+    launch_early(k_velshoot_force, row_grid(d), kRowThreads, 0, s, dp, lv0, comp(B[cb], 0),
+                 comp(B[cb], 1), comp(B[cb], 2), f, d);
     AW_TRY(cudaGetLastError());
     AW_TRY(fluid_forward_field(c->plan, comp(f, 0), comp(f, 1), comp(f, 2), s));
     AW_TRY(fluid_solve(c->plan, 1, s));
@@ -1068,7 +1104,7 @@ cudaError_t ldmm_velshoot_iterate(LdmmCtx *c, const float *I0, const float *I1, 
   }
   // residual, image energy, its splat, K(grad(I0) splat), the update
   AW_TRY(launch_apply(I0, comp(B[cb], 0), comp(B[cb], 1), comp(B[cb], 2), img, d, 0.0f, s));
-  k_residual<<<row_grid(d), kRowThreads, 0, s>>>(img, I1, c->diff, c->partials, d);
+  launch_early(k_residual, row_grid(d), kRowThreads, 0, s, img, I1, c->diff, c->partials, d);
   AW_TRY(cudaGetLastError());
   k_record_energy<<<1, kRecThreads, 0, s>>>(c->partials, c->nparts, spprod, c->energy, c->count,
                                             c->cap);
@@ -1081,10 +1117,10 @@ cudaError_t ldmm_velshoot_iterate(LdmmCtx *c, const float *I0, const float *I1, 
     AW_TRY(fluid_inverse_store(c->plan, comp(f, 0), comp(f, 1), comp(f, 2), s));
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->plan.device);
-    k_max_disp<<<sms * 4, 256, 0, s>>>(comp(v0, 0), comp(v0, 1), comp(v0, 2), comp(f, 0),
-                                       comp(f, 1), comp(f, 2), n, c->sigma, c->maxbits);
+    launch_early(k_max_disp, dim3(sms * 4), 256, 0, s, comp(v0, 0), comp(v0, 1), comp(v0, 2),
+                 comp(f, 0), comp(f, 1), comp(f, 2), n, c->sigma, c->maxbits);
     AW_TRY(cudaGetLastError());
-    k_step_from_max<<<1, 1, 0, s>>>(c->maxbits, c->max_pert, c->step);
+    launch_early(k_step_from_max, dim3(1), 1, 0, s, c->maxbits, c->max_pert, c->step);
     AW_TRY(cudaGetLastError());
   } else {
     AW_TRY(fluid_inverse_axpby(c->plan, comp(v0, 0), comp(v0, 1), comp(v0, 2), c->step, c->sigma,
@@ -1176,16 +1212,18 @@ cudaError_t ldmm_adshoot_iterate(LdmmCtx *c, const float *I0, const float *I1, f
     AW_TRY(launch_compose_vh(vv, hh, oo, d, c->sp, 1, BG_PARTIAL_ZERO, nullptr, 1.0f, s));
     AW_TRY(splat_sort(c->adSort[t], oo[0], oo[1], oo[2], s));
     AW_TRY(splat_gather(c->adSort[t], alpha0, oo[0], oo[1], oo[2], A(t), 0.0f, s));
-    k_forward_step<false><<<grid, kRowThreads, 0, s>>>(
-        comp(P1(t - 1), 0), comp(P1(t - 1), 1), comp(P1(t - 1), 2), vv[0], vv[1], vv[2],
-        comp(P1(t), 0), comp(P1(t), 1), comp(P1(t), 2), I0, I(t), d, space_div(c->sp));
+    launch_early(k_forward_step<false>, grid, kRowThreads, 0, s, comp(P1(t - 1), 0),
+                 comp(P1(t - 1), 1), comp(P1(t - 1), 2), vv[0], vv[1], vv[2], comp(P1(t), 0),
+                 comp(P1(t), 1), comp(P1(t), 2), I0, I(t), d, space_div(c->sp));
     return cudaGetLastError();
   };
 
   // shooting
-  k_identity<<<grid, kRowThreads, 0, s>>>(comp(P0(0), 0), comp(P0(0), 1), comp(P0(0), 2), d);
+  launch_early(k_identity, grid, kRowThreads, 0, s, comp(P0(0), 0), comp(P0(0), 1), comp(P0(0), 2),
+               d);
   AW_TRY(cudaGetLastError());
-  k_identity<<<grid, kRowThreads, 0, s>>>(comp(P1(0), 0), comp(P1(0), 1), comp(P1(0), 2), d);
+  launch_early(k_identity, grid, kRowThreads, 0, s, comp(P1(0), 0), comp(P1(0), 1), comp(P1(0), 2),
+               d);
   AW_TRY(cudaGetLastError());
   AW_TRY(velocity(I0, alpha0, 0));
   for (int t = 1; t < T; ++t) {
@@ -1198,14 +1236,14 @@ cudaError_t ldmm_adshoot_iterate(LdmmCtx *c, const float *I0, const float *I1, f
   // image term; v0 = -K f0 with f0 = grad(I0) alpha0, so L v0 = -f0 and the
   // product is formed from the force again (k_force_vdot), no second transform
   const double spprod = c->sp.x * c->sp.y * c->sp.z;
-  k_force_vdot<<<grid, kRowThreads, 0, s>>>(make_force(I0, alpha0, 0, c->sp), V(0), -1.0f,
+  launch_early(k_force_vdot, grid, kRowThreads, 0, s, make_force(I0, alpha0, 0, c->sp), V(0), -1.0f,
                                              c->partials, d);
   AW_TRY(cudaGetLastError());
   k_record_energy<<<1, kRecThreads, 0, s>>>(c->partials, c->nparts, spprod, c->venergy,
                                             c->count, c->cap, 0);
   AW_TRY(cudaGetLastError());
   const float inv = 1.0f / (c->sigma * c->sigma);
-  k_ad_residual<<<grid, kRowThreads, 0, s>>>(I(T), I1, inv, IHat, c->partials, d);
+  launch_early(k_ad_residual, grid, kRowThreads, 0, s, I(T), I1, inv, IHat, c->partials, d);
   AW_TRY(cudaGetLastError());
   k_record_energy<<<1, kRecThreads, 0, s>>>(c->partials, c->nparts, spprod, c->energy,
                                             c->count, c->cap, 1);
@@ -1220,28 +1258,28 @@ cudaError_t ldmm_adshoot_iterate(LdmmCtx *c, const float *I0, const float *I1, f
     const int t = i + 1;
     float *p0[3] = {comp(P0(t), 0), comp(P0(t), 1), comp(P0(t), 2)};
     float *p1[3] = {comp(P1(t), 0), comp(P1(t), 1), comp(P1(t), 2)};
-    k_ad_pull<false><<<grid, kRowThreads, 0, s>>>(aTil, p1[0], p1[1], p1[2], aHat, d);
+    launch_early(k_ad_pull<false>, grid, kRowThreads, 0, s, aTil, p1[0], p1[1], p1[2], aHat, d);
     AW_TRY(cudaGetLastError());
     AW_TRY(splat_gather(c->adSort[t], ITil, p0[0], p0[1], p0[2], IHat, 0.0f, s));
-    k_ad_force<<<grid, kRowThreads, 0, s>>>(aHat, A(t), I(t), IHat, comp(c->u, 0), comp(c->u, 1),
-                                            comp(c->u, 2), d, g);
+    launch_early(k_ad_force, grid, kRowThreads, 0, s, aHat, A(t), I(t), IHat, comp(c->u, 0),
+                 comp(c->u, 1), comp(c->u, 2), d, g);
     AW_TRY(cudaGetLastError());
     AW_TRY(fluid_forward_field(c->plan, comp(c->u, 0), comp(c->u, 1), comp(c->u, 2), s));
     AW_TRY(fluid_solve(c->plan, 1, s));
     AW_TRY(fluid_inverse_store(c->plan, comp(c->u, 0), comp(c->u, 1), comp(c->u, 2), s));
-    k_ad_dot_div<<<grid, kRowThreads, 0, s>>>(I(t), comp(c->u, 0), comp(c->u, 1), comp(c->u, 2),
-                                              A(t), s1, s2, d, g);
+    launch_early(k_ad_dot_div, grid, kRowThreads, 0, s, I(t), comp(c->u, 0), comp(c->u, 1),
+                 comp(c->u, 2), A(t), s1, s2, d, g);
     AW_TRY(cudaGetLastError());
-    k_ad_pull<true><<<grid, kRowThreads, 0, s>>>(s1, p0[0], p0[1], p0[2], aTil, d);
+    launch_early(k_ad_pull<true>, grid, kRowThreads, 0, s, s1, p0[0], p0[1], p0[2], aTil, d);
     AW_TRY(cudaGetLastError());
     if (t == T)
       AW_TRY(splat_gather(c->adSort[0], s2, p1[0], p1[1], p1[2], s1, 0.0f, s));
     else
       AW_TRY(splat(c->sw, s2, p1[0], p1[1], p1[2], s1, 0.0f, s));
-    k_ad_add<<<flat, 256, 0, s>>>(ITil, s1, n);
+    launch_early(k_ad_add, dim3(flat), 256, 0, s, ITil, s1, n);
     AW_TRY(cudaGetLastError());
   }
-  k_ad_alpha<<<grid, kRowThreads, 0, s>>>(I0, V(0), aTil, c->step, alpha0, d, g);
+  launch_early(k_ad_alpha, grid, kRowThreads, 0, s, I0, V(0), aTil, c->step, alpha0, d, g);
   AW_TRY(cudaGetLastError());
   // the data's maps end at t_1, where the reference's backward sweep leaves them
   AW_TRY(cudaMemcpyAsync(phi0T, P0(1), sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, s));
@@ -1282,27 +1320,28 @@ cudaError_t ldmm_iterate_orig(LdmmCtx *c, const float *I0, const float *I1, floa
   const DivD a2 = make_div(2.0 * c->sp.x), b2 = make_div(2.0 * c->sp.y), e2 = make_div(2.0 * c->sp.z);
   const DivD a1 = make_div(c->sp.x), b1 = make_div(c->sp.y), e1 = make_div(c->sp.z);
   // backward sweep: h <- h(x + v_t/sp), JT_t = I1(h), Jacobian transport
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(comp(H[0], 0), comp(H[0], 1), comp(H[0], 2), d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, comp(H[0], 0), comp(H[0], 1),
+               comp(H[0], 2), d);
   AW_TRY(cudaGetLastError());
   int cur = 0;
   for (int t = T - 1; t >= 0; --t) {
     float *vt = v + (long)t * 3 * n;
-    k_forward_step<true><<<row_grid(d), kRowThreads, 0, s>>>(
-        comp(H[cur], 0), comp(H[cur], 1), comp(H[cur], 2), comp(vt, 0), comp(vt, 1), comp(vt, 2),
-        comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I1, c->JT + (long)t * n,
-        d, space_div(c->sp));
+    launch_early(k_forward_step<true>, row_grid(d), kRowThreads, 0, s, comp(H[cur], 0),
+                 comp(H[cur], 1), comp(H[cur], 2), comp(vt, 0), comp(vt, 1), comp(vt, 2),
+                 comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I1,
+                 c->JT + (long)t * n, d, space_div(c->sp));
     AW_TRY(cudaGetLastError());
     cur = 1 - cur;
-    k_jacdet<<<row_grid(d), kRowThreads, 0, s>>>(comp(vt, 0), comp(vt, 1), comp(vt, 2),
-                                                 t == T - 1 ? nullptr : c->JD + (long)(t + 1) * n,
-                                                 c->JD + (long)t * n, d, space_div(c->sp), a2, b2, e2, a1, b1,
-                                                 e1);
+    launch_early(k_jacdet, row_grid(d), kRowThreads, 0, s, comp(vt, 0), comp(vt, 1), comp(vt, 2),
+                 t == T - 1 ? nullptr : c->JD + (long)(t + 1) * n, c->JD + (long)t * n, d,
+                 space_div(c->sp), a2, b2, e2, a1, b1, e1);
     AW_TRY(cudaGetLastError());
   }
   if (update_step) AW_TRY(cudaMemsetAsync(c->maxbits, 0, sizeof(unsigned), s));
   // forward sweep: S = I0(h), force grad(S) * (S - JT_t) * JacDet_t, K, update,
   // h <- h(x - v_t/sp) with the updated v_t, and S for the next t
-  k_identity<<<row_grid(d), kRowThreads, 0, s>>>(comp(H[0], 0), comp(H[0], 1), comp(H[0], 2), d);
+  launch_early(k_identity, row_grid(d), kRowThreads, 0, s, comp(H[0], 0), comp(H[0], 1),
+               comp(H[0], 2), d);
   AW_TRY(cudaGetLastError());
   cur = 0;
   float *Sb = c->S;
@@ -1315,27 +1354,28 @@ cudaError_t ldmm_iterate_orig(LdmmCtx *c, const float *I0, const float *I1, floa
       AW_TRY(fluid_inverse_store(c->plan, comp(c->u, 0), comp(c->u, 1), comp(c->u, 2), s));
       int sms = 148;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->plan.device);
-      k_max_disp<<<sms * 4, 256, 0, s>>>(comp(vt, 0), comp(vt, 1), comp(vt, 2), comp(c->u, 0),
-                                         comp(c->u, 1), comp(c->u, 2), n, c->sigma, c->maxbits);
+      launch_early(k_max_disp, dim3(sms * 4), 256, 0, s, comp(vt, 0), comp(vt, 1), comp(vt, 2),
+                   comp(c->u, 0), comp(c->u, 1), comp(c->u, 2), n, c->sigma, c->maxbits);
       AW_TRY(cudaGetLastError());
     } else {
       AW_TRY(fluid_inverse_axpby(c->plan, comp(vt, 0), comp(vt, 1), comp(vt, 2), c->step,
                                  c->sigma, s));
     }
-    k_forward_step<false><<<row_grid(d), kRowThreads, 0, s>>>(
-        comp(H[cur], 0), comp(H[cur], 1), comp(H[cur], 2), comp(vt, 0), comp(vt, 1), comp(vt, 2),
-        comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I0, Sb, d, space_div(c->sp));
+    launch_early(k_forward_step<false>, row_grid(d), kRowThreads, 0, s, comp(H[cur], 0),
+                 comp(H[cur], 1), comp(H[cur], 2), comp(vt, 0), comp(vt, 1), comp(vt, 2),
+                 comp(H[1 - cur], 0), comp(H[1 - cur], 1), comp(H[1 - cur], 2), I0, Sb, d,
+                 space_div(c->sp));
     AW_TRY(cudaGetLastError());
     cur = 1 - cur;
     // the image energy is recorded (and the count advanced) after the sweep
     if (c->vec_energy && !update_step) AW_TRY(vec_step_energy(c, vt, t, t == 0, 0, s));
   }
   if (update_step) {
-    k_step_from_max<<<1, 1, 0, s>>>(c->maxbits, c->max_pert, c->step);
+    launch_early(k_step_from_max, dim3(1), 1, 0, s, c->maxbits, c->max_pert, c->step);
     return cudaGetLastError();
   }
   // image energy of the updated path: sp^3 * sum (I0(h) - I1)^2
-  k_residual<<<row_grid(d), kRowThreads, 0, s>>>(Sb, I1, c->diff, c->partials, d);
+  launch_early(k_residual, row_grid(d), kRowThreads, 0, s, Sb, I1, c->diff, c->partials, d);
   AW_TRY(cudaGetLastError());
   const double spprod = c->sp.x * c->sp.y * c->sp.z;
   k_record_energy<<<1, kRecThreads, 0, s>>>(c->partials, c->nparts, spprod, c->energy,

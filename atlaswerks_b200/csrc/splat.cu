@@ -32,6 +32,7 @@ AW_D long bucket_of(const Dims &d, float px, float py, float pz) {
 __global__ void __launch_bounds__(kRowThreads)
     k_count(const float *__restrict__ hx, const float *__restrict__ hy, const float *__restrict__ hz,
             Dims d, int *__restrict__ counts, int *__restrict__ place) {
+  early_entry();
   Voxel v;
   if (!voxel_of(d, v)) return;
   const long b = bucket_of(d, hx[v.i], hy[v.i], hz[v.i]);
@@ -78,6 +79,7 @@ AW_D int block_scan(int (&a)[kScanItems], int *wsum) {
 
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_reduce(const int *__restrict__ x, long n, int *__restrict__ blocksums) {
+  early_entry();
   const long b0 = (long)blockIdx.x * kScanBlock;
   int s = 0;
   for (int k = 0; k < kScanItems; ++k) {
@@ -98,6 +100,7 @@ __global__ void __launch_bounds__(kScanThreads)
 
 // one block: exclusive scan of the block sums, chunk by chunk
 __global__ void __launch_bounds__(kScanThreads) k_scan_blocksums(int *__restrict__ bs, int nb) {
+  early_entry();
   __shared__ int wsum[kScanThreads / 32 + 1];
   int carry = 0;
   for (int c0 = 0; c0 < nb; c0 += kScanBlock) {
@@ -118,9 +121,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_blocksums(int *__restrict
   }
 }
 
-// exclusive scan in place; x[n] receives the total
+// exclusive scan in place; x[n] receives the total. SUM: blocksums holds the
+// blocks' own sums, and each block adds up those before it (up to kScanSum of
+// them: a 16 KB read from L2 against a launch of its own for their scan).
+constexpr int kScanSum = 4096;
+template <bool SUM>
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_apply(int *__restrict__ x, long n, const int *__restrict__ blocksums) {
+  early_entry();
   __shared__ int wsum[kScanThreads / 32 + 1];
   const long b0 = (long)blockIdx.x * kScanBlock;
   int a[kScanItems];
@@ -130,7 +138,20 @@ __global__ void __launch_bounds__(kScanThreads)
     a[k] = i < n ? x[i] : 0;
   }
   const int total = block_scan(a, wsum);
-  const int off = blocksums[blockIdx.x];
+  int off = 0;
+  if (SUM) {
+    for (int j = threadIdx.x; j < (int)blockIdx.x; j += kScanThreads) off += blocksums[j];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) off += __shfl_xor_sync(0xffffffffu, off, o);
+    __syncthreads();  // block_scan's use of wsum is over
+    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = off;
+    __syncthreads();
+    off = 0;
+#pragma unroll
+    for (int w = 0; w < kScanThreads / 32; ++w) off += wsum[w];
+  } else {
+    off = blocksums[blockIdx.x];
+  }
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     const long i = b0 + (long)threadIdx.x * kScanItems + k;
@@ -169,6 +190,7 @@ __global__ void __launch_bounds__(kRowThreads)
     k_scatter(const float *__restrict__ hx, const float *__restrict__ hy,
               const float *__restrict__ hz, Dims d, const int *__restrict__ offsets,
               const int *__restrict__ place, int *__restrict__ order) {
+  early_entry();
   Voxel v;
   if (!voxel_of(d, v)) return;
   const long b = bucket_of(d, hx[v.i], hy[v.i], hz[v.i]);
@@ -285,6 +307,7 @@ AW_D void block_radix_sort(int *__restrict__ order, int *__restrict__ tmp, int s
 __global__ void __launch_bounds__(kSortThreads)
     k_bucket_sort(const int *__restrict__ offsets, int *__restrict__ order, int *__restrict__ tmp,
                   long next, long n) {
+  early_entry();
   __shared__ SortShared sh;
   // the sums' queue (tmp's first n places, then its count and the blocks
   // done with it) starts empty
@@ -325,6 +348,7 @@ __global__ void __launch_bounds__(256)
                const float *__restrict__ img, const float *__restrict__ hx,
                const float *__restrict__ hy, const float *__restrict__ hz,
                float *__restrict__ prod) {
+  early_entry();
   const int p = blockIdx.x * 256 + threadIdx.x;
   if (p >= *total) return;
   const int m = order[p];
@@ -462,6 +486,7 @@ AW_D void first_products(const GatherArgs &a, const Ranges &q, const int *m, flo
 
 template <bool PRE>
 __global__ void __launch_bounds__(kGatherThreads) k_gather(const __grid_constant__ GatherArgs a) {
+  early_entry();
   const int i = blockIdx.x * kGatherThreads + threadIdx.x;
   bool later = false;
   if (i < a.n) {
@@ -511,6 +536,7 @@ AW_D void rank_pair(unsigned (&rk)[2], const int *m, int i, int j) {
 // the queue for the next image splatted by the same map
 template <bool PRE>
 __global__ void __launch_bounds__(kQueuedThreads) k_gather_queued(const __grid_constant__ GatherArgs a) {
+  early_entry();
   __shared__ float byrank[kSlots][kQueuedThreads];
   const int tid = threadIdx.x, count = *(volatile int *)(a.queue + a.n);
   for (int t = blockIdx.x * kQueuedThreads + tid; t < count; t += gridDim.x * kQueuedThreads) {
@@ -606,13 +632,20 @@ cudaError_t splat_sort(const SplatWork &w, const float *hx, const float *hy, con
   const Dims d = w.d;
   cudaError_t e;
   if ((e = cudaMemsetAsync(w.offsets, 0, sizeof(int) * (w.next + 1), s)) != cudaSuccess) return e;
-  k_count<<<row_grid(d), kRowThreads, 0, s>>>(hx, hy, hz, d, w.offsets, w.cursor);
-  k_scan_reduce<<<w.nblocks, kScanThreads, 0, s>>>(w.offsets, w.next, w.blocksums);
-  k_scan_blocksums<<<1, kScanThreads, 0, s>>>(w.blocksums, w.nblocks);
-  k_scan_apply<<<w.nblocks, kScanThreads, 0, s>>>(w.offsets, w.next, w.blocksums);
-  k_scatter<<<row_grid(d), kRowThreads, 0, s>>>(hx, hy, hz, d, w.offsets, w.cursor, w.order);
-  k_bucket_sort<<<(int)((w.next + kSortThreads - 1) / kSortThreads), kSortThreads, 0, s>>>(
-      w.offsets, w.order, w.cursor, w.next, d.n());
+  launch_early(k_count, row_grid(d), kRowThreads, 0, s, hx, hy, hz, d, w.offsets, w.cursor);
+  launch_early(k_scan_reduce, dim3(w.nblocks), kScanThreads, 0, s, w.offsets, w.next, w.blocksums);
+  if (w.nblocks <= kScanSum) {
+    launch_early(k_scan_apply<true>, dim3(w.nblocks), kScanThreads, 0, s, w.offsets, w.next,
+                 w.blocksums);
+  } else {
+    launch_early(k_scan_blocksums, dim3(1), kScanThreads, 0, s, w.blocksums, w.nblocks);
+    launch_early(k_scan_apply<false>, dim3(w.nblocks), kScanThreads, 0, s, w.offsets, w.next,
+                 w.blocksums);
+  }
+  launch_early(k_scatter, row_grid(d), kRowThreads, 0, s, hx, hy, hz, d, w.offsets, w.cursor,
+               w.order);
+  launch_early(k_bucket_sort, dim3((int)((w.next + kSortThreads - 1) / kSortThreads)), kSortThreads,
+               0, s, w.offsets, w.order, w.cursor, w.next, d.n());
   return cudaGetLastError();
 }
 
@@ -625,13 +658,13 @@ cudaError_t splat_gather(const SplatWork &w, const float *img, const float *hx, 
   // seven blocks an SM, or one thread per destination
   const unsigned queued = (unsigned)std::min<long>((d.n() + kQueuedThreads - 1) / kQueuedThreads, 7 * 148);
   if (w.prod) {
-    k_products<<<(unsigned)((d.n() + 255) / 256), 256, 0, s>>>(w.order, w.offsets + w.next, d.n(), img,
-                                                               hx, hy, hz, w.prod);
-    k_gather<true><<<grid, kGatherThreads, 0, s>>>(a);
-    k_gather_queued<true><<<queued, kQueuedThreads, 0, s>>>(a);
+    launch_early(k_products, dim3((unsigned)((d.n() + 255) / 256)), 256, 0, s, w.order,
+                 w.offsets + w.next, d.n(), img, hx, hy, hz, w.prod);
+    launch_early(k_gather<true>, dim3(grid), kGatherThreads, 0, s, a);
+    launch_early(k_gather_queued<true>, dim3(queued), kQueuedThreads, 0, s, a);
   } else {
-    k_gather<false><<<grid, kGatherThreads, 0, s>>>(a);
-    k_gather_queued<false><<<queued, kQueuedThreads, 0, s>>>(a);
+    launch_early(k_gather<false>, dim3(grid), kGatherThreads, 0, s, a);
+    launch_early(k_gather_queued<false>, dim3(queued), kQueuedThreads, 0, s, a);
   }
   return cudaGetLastError();
 }

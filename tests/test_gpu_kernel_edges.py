@@ -76,6 +76,16 @@ def test_splat_candidate_counts(oracle, shape, scale, jitter):
         assert np.array_equal(host(D.splat(cu(img), cu(h), 0.25)), want)
 
 
+@pytest.mark.parametrize("shape", [(1, 2, 340), (160, 160, 160), (160, 161, 160)])
+def test_splat_scan_sizes(oracle, shape):
+    """Cells of two blocks of the scan, and just below and above the most
+    whose sums its last kernel adds up itself (4096 blocks of 1024)."""
+    rng = np.random.default_rng(37)
+    img = rng.normal(0, 1, shape).astype(np.float32)
+    h = (identity(shape) + rng.normal(0, 0.4, (3,) + shape)).astype(np.float32)
+    assert np.array_equal(host(D.splat(cu(img), cu(h), 0.0)), oracle.splat(img, h, 0.0))
+
+
 @pytest.mark.parametrize("grid", [(1, 8, 32, 16), (2, 6, 32, 24), (1, 3, 32, 16), (1, 32, 64, 64)])
 @pytest.mark.parametrize("cin,cout", [(16, 16), (48, 16), (16, 32), (32, 32)])
 @pytest.mark.parametrize("masked", [True, False])
