@@ -91,11 +91,17 @@ AW_D uint32_t mnmajor_off(int k, int c, int R) { return (k >> 3) * (R * 16) + c 
 // ---- operand loaders ----------------------------------------------------------
 // Each loader copies this thread's 16-byte chunks of one 64-deep K step
 // from global memory straight into the stage's canonical layout with
-// cp.async (zero-filled past kend or outside the volume; cached in L1, where
-// the 27 taps of neighbouring rows meet); init() computes the per-thread
-// context once per CTA.
+// cp.async (zero-filled past kend or outside the volume); init() computes the
+// per-thread context once per CTA. cp_async16 keeps the lines in L1, for the
+// weights and for the weight gradient, whose rows re-read them (its 16-column
+// GEMM at 64^3 takes 47 us so, 86 past L1); cp_async16_l2 passes L1 by.
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc, bool valid) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)),
+               "l"(gsrc), "r"(valid ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async16_l2(void *smem_dst, const void *gsrc, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)),
                "l"(gsrc), "r"(valid ? 16 : 0)
                : "memory");
 }
@@ -108,10 +114,17 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // A of forward / dgrad: rows = voxels, K = (tap, channel) of X shifted by
-// sign * off(tap); K-major (the 8 channels of a chunk are contiguous).
-// Thread t owns row t of the tile; which taps stay inside the volume for
-// that voxel is a 27-bit mask, and the voxel-index offset of each tap a
-// table in shared memory, both made once per CTA.
+// sign * off(tap); K-major (the 8 channels of a chunk are contiguous). Which
+// taps stay inside the volume for a row's voxel is a 27-bit mask, the
+// voxel-index offset of each tap a second table, both made once per CTA in
+// shared memory. The L1 / shared-memory data pipe bounds these GEMMs (73 % of
+// its peak over the 96 -> 32 layer at 32^3, 90 % while its CTAs run, the
+// tensor pipe idle), so the copies pass L1 by and a warp's take 8 rows x 4
+// chunks at a time, 64 contiguous bytes a row. Against one row a thread
+// through L1: 96 -> 32 at 32^3 67.9 -> 64.4 us (the tensor work of it takes
+// 3.4), the 64-column layers at 16^3
+// 18.0 -> 14.4, the 128-column ones at 8^3 9.1 -> 8.9, 16 -> 16 with one tap
+// at 64^3 15.2 -> 16.0.
 struct LoadConvA {
   const bf16 *x;
   Vol v;
@@ -120,53 +133,58 @@ struct LoadConvA {
   FastDiv fc;
   static constexpr int kMN = 0;
   struct Ctx {
-    int m;
-    uint32_t vmask;
+    int m0;
+    const uint32_t *vmask;
     const int *toff;
   };
   AW_D Ctx init(long m0) const {
     __shared__ int s_toff[27];
+    __shared__ uint32_t s_vmask[kGBM];
     if (threadIdx.x < ntaps) {
       int dz, dy, dx;
       tap_offset(threadIdx.x, ntaps, dz, dy, dx);
       s_toff[threadIdx.x] = sign * ((dz * v.H + dy) * v.W + dx);
     }
-    Ctx c;
-    c.m = (int)m0 + threadIdx.x;
-    c.toff = s_toff;
-    c.vmask = 0;
-    if (c.m < M) {
+    const int m = (int)m0 + threadIdx.x;
+    uint32_t mask = 0;
+    if (m < M) {
       int b, z, y, xx;
-      voxel_coords(v, c.m, b, z, y, xx);
+      voxel_coords(v, m, b, z, y, xx);
       for (int t = 0; t < ntaps; ++t) {
         int dz, dy, dx;
         tap_offset(t, ntaps, dz, dy, dx);
         const int zz = z + sign * dz, yy = y + sign * dy, xs = xx + sign * dx;
-        if (zz >= 0 && zz < v.D && yy >= 0 && yy < v.H && xs >= 0 && xs < v.W) c.vmask |= 1u << t;
+        if (zz >= 0 && zz < v.D && yy >= 0 && yy < v.H && xs >= 0 && xs < v.W) mask |= 1u << t;
       }
     }
-    return c;  // the caller synchronises the CTA before the first issue()
+    s_vmask[threadIdx.x] = mask;
+    return Ctx{(int)m0, s_vmask, s_toff};  // the caller synchronises the CTA before the first issue()
   }
   AW_D void issue(const Ctx &c, uint8_t *s, int k0, int kend) const {
-    int tap = (int)fc.div((uint32_t)k0);
-    int ci = k0 - tap * C;
+    static_assert(kGThreads == 128 && kGBM == 128 && kGBK == 64, "copy layout");
+    const int j0 = threadIdx.x & 3, r0 = threadIdx.x >> 2;
+    uint32_t vm[4];
 #pragma unroll
-    for (int j = 0; j < kGBK / 8; ++j) {
-      const bool ok = ((c.vmask >> tap) & 1u) && (k0 + 8 * j < kend);
-      const bf16 *src = ok ? x + (long)(c.m + c.toff[tap]) * C + ci : x;
-      cp_async16(s + kmajor_off(threadIdx.x, j, kGBM), src, ok);
-      ci += 8;
-      if (ci == C) {
-        ci = 0;
-        ++tap;
+    for (int i = 0; i < 4; ++i) vm[i] = c.vmask[r0 + 32 * i];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int j = j0 + 4 * h, k = k0 + 8 * j;
+      const bool kin = k < kend;
+      const int tap = kin ? (int)fc.div((uint32_t)k) : 0, ci = k - tap * C;
+      const bf16 *row = x + (long)(c.m0 + r0 + c.toff[tap]) * C + ci;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const bool ok = kin && ((vm[i] >> tap) & 1u);
+        cp_async16_l2(s + kmajor_off(r0 + 32 * i, j, kGBM), ok ? row + (long)(32 * i) * C : x, ok);
       }
     }
   }
 };
 
 // B of forward / dgrad: rows = output columns n < N, K contiguous per row.
-// Chunk i = tid + 128 q: row i / 8, K chunk i % 8 (8 threads read one
-// row's 128 contiguous bytes).
+// Chunk i = tid + 128 q: K chunk i % 4 of row i / 4, then chunks 4 to 7 (four
+// threads read 64 contiguous bytes of a row; with eight of a row a warp's
+// chunks met in half of the banks, 96 -> 32 at 32^3 64.4 against 61.4 us).
 template <int BN>
 struct LoadRowsB {
   const bf16 *w;  // [BN][K]
@@ -179,7 +197,7 @@ struct LoadRowsB {
 #pragma unroll
     for (int q = 0; q < kChunks; ++q) {
       const int i = threadIdx.x + kGThreads * q;
-      const int row = i >> 3, j = i & 7, k = k0 + 8 * j;
+      const int row = (i >> 2) % BN, j = (i & 3) + 4 * ((i >> 2) / BN), k = k0 + 8 * j;
       const bool ok = k < kend;
       cp_async16(s + kmajor_off(row, j, BN), ok ? w + (long)row * K + k : w, ok);
     }
@@ -995,7 +1013,7 @@ __global__ void __launch_bounds__(128)
   }
   // weights [COUT][27][CIN] -> chunk (tap, j, n) at ((tap*NCH + j)*(COUT/8) + n/8)*128 +
   // (n%8)*16 = 16 c for c = (tap*NCH + j)*COUT + n: consecutive threads, consecutive chunks
-#pragma unroll 1
+#pragma unroll 8
   for (int c = tid; c < COUT * 27 * C::NCH; c += 128) {
     const int n = c % COUT, r = c / COUT;
     const int j = r % C::NCH, tap = r / C::NCH;
