@@ -12,8 +12,10 @@
 //               complex-to-real along x -> consumer epilogue (store, or the
 //               LDMM velocity update).
 //
-// The half spectrum (3 x nz x ny x (nx/2+1) complex64) makes two HBM round
-// trips instead of the six of a pass-per-axis transform.
+// The half spectrum (3 x nz x ny x (nx/2+1) complex64, or the slabs that
+// fluid_any.cuh describes) makes two HBM round trips instead of the six of
+// a pass-per-axis transform. fluid_fast.cu has the kernels for axes that
+// are powers of two in [16, 256], fluid_any.cu those for any other grid.
 #pragma once
 
 #include <cuda.h>

@@ -1,7 +1,7 @@
 // fluid_fast.cu — the fluid-operator kernels for power-of-two axes
 // (16..256), with register-resident line FFTs (fft_reg.cuh).
 //
-// Same three passes as fluid.cu (xy-forward, z-solve, xy-inverse) and the
+// Same three passes as fluid_any.cu (xy-forward, z-solve, xy-inverse) and the
 // same arithmetic definition; the layout of work differs:
 //  * xy kernels: one 256-thread CTA per (z-slab, component) holding only the
 //    slab's half spectrum in shared memory (66.5 KB at 128 x 128, three

@@ -13,9 +13,10 @@
 //
 // plus, at a step-size update (iteration 0 of a scale level,
 // GreedyWarp.txx:99), a max|v| reduction and eps = MaxPert / max|v| computed
-// on the device (GreedyIteratorCPU.cxx:125-131). On the register-FFT path,
-// iterations without a step update or an inverse field run 5 and 6 as one
-// kernel (k_xy_inv_compose, fluid_fast.cu): five launches.
+// on the device (GreedyIteratorCPU.cxx:125-131). On small grids of the
+// register-FFT path, iterations without a step update or an inverse field
+// run 5 and 6 as one kernel (k_xy_inv_compose, fluid_fast.cu; the limit and
+// its reason are at kFuseVoxels): five launches.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -142,9 +143,6 @@ __global__ void k_set_step(const unsigned *__restrict__ maxbits, float max_pert,
   *step = fdiv(max_pert, __uint_as_float(*maxbits));
 }
 
-// composeHV(h, eps*v, PARTIAL_ID) and, when hinv is given,
-// composeVHInv(eps*v, hinv, PARTIAL_ZERO) — GreedyIteratorCPU::updateDeformation
-// (GreedyIteratorCPU.cxx:83-95), both from one read of v.
 // composeHV(h, eps*v, PARTIAL_ID) and, when hinv is given,
 // composeVHInv(eps*v, hinv, PARTIAL_ZERO) — GreedyIteratorCPU::updateDeformation
 // (GreedyIteratorCPU.cxx:83-95), both from one read of v. q[] divides by the
@@ -622,8 +620,8 @@ cudaError_t greedy_stage(GreedyCtx *g, int stage, const float *I0, const float *
 // it joins before the step-size stage and the update, the two readers and
 // writers of the step it may reduce (AutoStepReduce).
 //
-// Without a step-size update or an inverse field, on the register-FFT path,
-// the inverse transform and the update are one kernel (kStageInvCompose):
+// Without a step-size update or an inverse field, on the register-FFT path
+// up to kFuseVoxels, the inverse transform and the update are one kernel (kStageInvCompose):
 // v = K f stays in shared memory. The step update needs max |v| over the
 // whole field before any voxel moves, and the inverse field gathers v at
 // h^-1(x) anywhere in the volume, so those iterations store v.

@@ -6,9 +6,10 @@
 // contributions in source (z, y, x) order, in float; the reference GPU path
 // uses int32 fixed-point atomics (CUDACommon/src/cudaSplatAtomic.cu:379-448).
 // Here the sources are bucketed by the cell their h lands in (counting sort:
-// count, exclusive scan, scatter, per-bucket sort by source index), then
-// every destination voxel merges the eight buckets that can reach it in
-// source-index order and adds the contributions sequentially. No float
+// count, exclusive scan, scatter, per-bucket sort by source index), their
+// eight contributions are formed once each, and every destination voxel adds
+// those of the eight buckets that can reach it sequentially in source-index
+// order (how it finds that order depends on their number, splat.cu). No float
 // atomics, run-to-run bitwise identical, and with identical inputs bitwise
 // equal to the reference CPU.
 #pragma once

@@ -14,7 +14,7 @@
  *
  * Grid limits: every axis in [2, 512] (the reference caps FFT axes at 512,
  * CUDACommon/src/cudaFFTSolver.cu:21). Slabs whose half spectrum,
- * ny*(nx/2+1)*8 bytes plus batch buffers, fits one CTA's shared memory
+ * ny*(nx/2+1)*8 bytes and a margin, fits one CTA's shared memory
  * (227 KB, e.g. up to 224 x 224) are transformed in x and y by one kernel;
  * larger ones (256 x 256, 512 x 512, ...) by an x pass and a y pass through
  * the spectrum in device memory, with the same arithmetic.
@@ -157,9 +157,11 @@ int aw_fluid_create(int nx, int ny, int nz, double spx, double spy, double spz, 
  * ApplyOperator (v <- L v). */
 int aw_fluid_apply(aw_fluid_t k, float *vx, float *vy, float *vz, int inverse, void *stream);
 int aw_fluid_destroy(aw_fluid_t k);
-/* Launch shapes of the shared-memory FFT path (grids with an axis that is
- * not a power of two in [16, 256]): x-line pairs per batch, y-columns per
- * batch, (ky,kx) columns per z-pass CTA. The plan autotunes them when it is
+/* Launch shapes of the any-size path (grids with an axis that is not a
+ * power of two in [16, 256]): row pairs per x-pass CTA and columns per
+ * y-pass CTA, which only grids whose slabs exceed one CTA's shared memory
+ * use, and (ky,kx) columns per z-pass CTA, taken as the next of 8, 16 and
+ * 32. The plan autotunes them when it is
  * created (each candidate timed on the device; the choice is kept per grid
  * and device for the process); aw_fluid_autotune re-runs the tuning,
  * aw_fluid_set_shapes overrides it. Results do not depend on the shapes.
@@ -209,14 +211,16 @@ int aw_greedy_set_auto_step_reduce(aw_greedy_t g, int on);
  * Both give the same bits; the switch exists to compare them. */
 int aw_greedy_set_staged_update(aw_greedy_t g, int on);
 /* on = 1 (default): an iteration without a step-size update or an inverse
- * field, on a grid of power-of-two axes, runs the inverse transform and the
- * update h' = h(x + eps v/sp) as one kernel, so v = K f never goes to HBM
- * (the stages GreedyIteratorGPU::Iterate runs as cplFFT inverse and
- * composeHV, Greedy/GreedyIteratorGPU.cxx:120-134); 0: v is stored and the
- * update is a kernel of its own. Both give the same bits. */
+ * field, on a grid of power-of-two axes smaller than 64^3 voxels, runs the
+ * inverse transform and the update h' = h(x + eps v/sp) as one kernel, so
+ * v = K f never goes to HBM (the stages GreedyIteratorGPU::Iterate runs as
+ * cplFFT inverse and composeHV, Greedy/GreedyIteratorGPU.cxx:120-134); 0,
+ * and on larger grids, where it is faster: v is stored and the update is a
+ * kernel of its own. Both give the same bits. */
 int aw_greedy_set_fused_update(aw_greedy_t g, int on);
-/* on = 1: I0(h) in the force preparation and h(x + eps v/sp) in the fused
- * update interpolate with float fused multiply-adds instead of the
+/* on = 1: I0(h) in the force preparation and h(x + eps v/sp) in the update
+ * of an iteration that set_fused_update covers (power-of-two axes of any
+ * size, no step update, no inverse field) interpolate with float fused multiply-adds instead of the
  * reference's double weights and sums: a few float ulps from the
  * bit-exact results (I0(h) within 1e-6 of it for images in [0, 1]); 0
  * (default): bit-exact with the reference CPU's interpolation. */
@@ -247,7 +251,8 @@ int aw_greedy_run(aw_greedy_t g, const float *I0, const float *I1, float *hx, fl
 
 /* Per-kernel device time of one iteration: each stage (0 force-prep,
  * 1 energy, 2 xy-forward FFT, 3 z-solve, 4 xy-inverse FFT, 5 max-norm,
- * 6 update, 7 xy-inverse FFT fused with the update) is launched `reps` times
+ * 6 update, 7 xy-inverse FFT fused with the update, or stages 4 and 6 where
+ * an iteration runs those) is launched `reps` times
  * back to back between CUDA events on `stream`; ms_out[8] receives the mean
  * milliseconds per launch. Leaves h_out holding one iteration's result;
  * records extra energies. Synchronises. */
