@@ -761,40 +761,70 @@ __global__ void k_sum_partials(const double *__restrict__ p, int n, double scale
   }
 }
 
-// dW = sum over K splits of the partials [split][co][K]: 64 sums a block,
-// each by four threads over a quarter of the splits
-constexpr int kReduceOuts = 64;
+// out[i] = part[0][i] + part[1][i] + ..., rows added in their order (FP32, one
+// accumulator): the weight gradients' K splits and the bias gradients'
+// blocks. Enough sums to fill the GPU: one a thread, 16 loads in flight.
 __global__ void __launch_bounds__(kEw)
-    k_reduce_splits(const float *__restrict__ part, int splits, long n, float *__restrict__ dw) {
-  constexpr int Q = kEw / kReduceOuts;
-  __shared__ float sh[Q][kReduceOuts];
-  const int o = threadIdx.x % kReduceOuts, q = threadIdx.x / kReduceOuts;
-  const long i = (long)blockIdx.x * kReduceOuts + o;
+    k_sum_rows(const float *__restrict__ part, int rows, long n, float *__restrict__ out) {
+  const long i = (long)blockIdx.x * kEw + threadIdx.x;
+  if (i >= n) return;
   float s = 0.0f;
-  if (i < n) {
-#pragma unroll 8
-    for (int k = q; k < splits; k += Q) s += part[k * n + i];
-  }
-  sh[q][o] = s;
-  __syncthreads();
-  if (q == 0 && i < n) {
-    float t = sh[0][o];
+#pragma unroll 16
+  for (int r = 0; r < rows; ++r) s += part[r * n + i];
+  out[i] = s;
+}
+// Few long sums: a block takes 32 of them, all its warps fetch 256 rows, and
+// the next 256 while one warp adds those in shared memory.
+constexpr int kSumCols = 32, kSumRows = 256, kSumThreads = 1024;
+__global__ void __launch_bounds__(kSumThreads)
+    k_sum_rows_staged(const float *__restrict__ part, int rows, long n, float *__restrict__ out) {
+  constexpr int W = kSumThreads / kSumCols, U = kSumRows / W;
+  __shared__ float sh[kSumRows][kSumCols];
+  const int c = threadIdx.x % kSumCols, w = threadIdx.x / kSumCols;
+  const long i = (long)blockIdx.x * kSumCols + c;
+  float v[U];
+  auto fetch = [&](int r0) {
 #pragma unroll
-    for (int w = 1; w < Q; ++w) t += sh[w][o];
-    dw[i] = t;
+    for (int u = 0; u < U; ++u) {
+      const int r = r0 + w + u * W;
+      v[u] = i < n && r < rows ? part[r * n + i] : 0.0f;
+    }
+  };
+  fetch(0);
+  float s = 0.0f;
+  for (int r0 = 0; r0 < rows; r0 += kSumRows) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) sh[w + u * W][c] = v[u];
+    __syncthreads();
+    fetch(r0 + kSumRows);
+    if (w == 0) {
+      const int m = min(kSumRows, rows - r0);
+#pragma unroll 16
+      for (int r = 0; r < m; ++r) s += sh[r][c];
+    }
+    __syncthreads();
   }
+  if (w == 0 && i < n) out[i] = s;
+}
+// The line: one sum a thread leaves most of the GPU idle below some 32768
+// sums and waits for memory once every 16 rows (20736 sums of 108 rows: 9.0
+// us, staged 5.6); with few rows a staged block has almost nothing to fetch
+// (110592 sums of 8 rows: 36 us staged, by 256 threads, against 3.1).
+constexpr long kStagedSums = 32768;
+constexpr int kStagedRows = 32;
+inline void sum_rows(const float *part, int rows, long n, float *out, cudaStream_t s) {
+  if (n < kStagedSums && rows > kStagedRows)
+    k_sum_rows_staged<<<(unsigned)((n + kSumCols - 1) / kSumCols), kSumThreads, 0, s>>>(part, rows, n, out);
+  else
+    k_sum_rows<<<ew_grid(n), kEw, 0, s>>>(part, rows, n, out);
 }
 // bias gradient: column sums of dY [M][N]; block b sums rows
-// [b*kBiasRows, (b+1)*kBiasRows) into part[b][N], then one block adds the
-// partials in block order
+// [b*kBiasRows, (b+1)*kBiasRows) into part[b][N] (thread (n, g) every
+// kEw/N-th row from the g-th, then the groups in their order), sum_rows adds
+// the blocks in theirs
 constexpr int kBiasRows = 512;
-__global__ void k_bias_partial(const bf16 *__restrict__ dy, long M, int N, float *__restrict__ part) {
+AW_D void bias_finish(float s, int N, float *__restrict__ part) {
   const int groups = kEw / N;
-  const int n = threadIdx.x % N, g = threadIdx.x / N;
-  const long r0 = (long)blockIdx.x * kBiasRows, r1 = min(M, r0 + kBiasRows);
-  float s = 0.0f;
-  if (g < groups)
-    for (long m = r0 + g; m < r1; m += groups) s += __bfloat162float(dy[m * N + n]);
   __shared__ float sh[kEw];
   sh[threadIdx.x] = s;
   __syncthreads();
@@ -804,50 +834,44 @@ __global__ void k_bias_partial(const bf16 *__restrict__ dy, long M, int N, float
     part[(long)blockIdx.x * N + threadIdx.x] = t;
   }
 }
-// the same, eight channels (16 bytes) a load, for N a multiple of 8 and 16-byte
-// aligned rows
+__global__ void k_bias_partial(const bf16 *__restrict__ dy, long M, int N, float *__restrict__ part) {
+  const int groups = kEw / N;
+  const int n = threadIdx.x % N, g = threadIdx.x / N;
+  const long r0 = (long)blockIdx.x * kBiasRows, r1 = min(M, r0 + kBiasRows);
+  float s = 0.0f;
+  if (g < groups)
+    for (long m = r0 + g; m < r1; m += groups) s += __bfloat162float(dy[m * N + n]);
+  bias_finish(s, N, part);
+}
+// the same sums in the same order, the rows fetched 16 bytes a load through
+// shared memory, 32 KB at a time (N a multiple of 8, 16-byte aligned rows)
+constexpr int kBiasTile = 16384;  // elements
 __global__ void __launch_bounds__(kEw)
     k_bias_partial8(const bf16 *__restrict__ dy, long M, int N, float *__restrict__ part) {
-  const int chunks = N / 8, groups = kEw / chunks;
-  const int c = threadIdx.x % chunks, g = threadIdx.x / chunks;
-  const long r0 = (long)blockIdx.x * kBiasRows, r1 = min(M, r0 + kBiasRows);
-  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (g < groups)
-#pragma unroll 4
-    for (long m = r0 + g; m < r1; m += groups) {
-      float f[8];
-      bf8_to_f(__ldg(reinterpret_cast<const uint4 *>(dy + m * N) + c), f);
+  __shared__ uint4 tile[kBiasTile / 8];
+  const int groups = kEw / N;
+  const int n = threadIdx.x % N, g = threadIdx.x / N;
+  const long r0 = (long)blockIdx.x * kBiasRows;
+  const int rows = (int)min(M - r0, (long)kBiasRows), step = kBiasTile / N;
+  const bf16 *t = reinterpret_cast<const bf16 *>(tile);
+  float s = 0.0f;
+  int m = g;  // the thread's next row
+  for (int p0 = 0; p0 < rows; p0 += step) {
+    const int p1 = min(rows, p0 + step), chunks = (p1 - p0) * N / 8;
+    const uint4 *src = reinterpret_cast<const uint4 *>(dy + (r0 + p0) * N);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) s[k] += f[k];
+    for (int u = 0; u < kBiasTile / 8 / kEw; ++u) {
+      const int i = threadIdx.x + u * kEw;
+      if (i < chunks) tile[i] = __ldg(src + i);
     }
-  __shared__ float sh[8][kEw];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) sh[k][threadIdx.x] = s[k];
-  __syncthreads();
-  if (threadIdx.x < N) {
-    const int k = threadIdx.x % 8, cc = threadIdx.x / 8;
-    float t = 0.0f;
-    for (int gg = 0; gg < groups; ++gg) t += sh[k][gg * chunks + cc];
-    part[(long)blockIdx.x * N + threadIdx.x] = t;
+    __syncthreads();
+    if (g < groups) {
+#pragma unroll 8
+      for (; m < p1; m += groups) s += __bfloat162float(t[(m - p0) * N + n]);
+    }
+    __syncthreads();
   }
-}
-// one block per channel: strided sums, then the warp and block trees (the
-// same order on every run)
-__global__ void __launch_bounds__(kEw)
-    k_bias_final(const float *__restrict__ part, int nb, int N, float *__restrict__ db) {
-  const int n = blockIdx.x;
-  float t = 0.0f;
-  for (int b = threadIdx.x; b < nb; b += kEw) t += part[(long)b * N + n];
-  __shared__ float sh[kEw / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float u = 0.0f;
-    for (int w = 0; w < kEw / 32; ++w) u += sh[w];
-    db[n] = u;
-  }
+  bias_finish(s, N, part);
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 masters
@@ -1234,6 +1258,16 @@ size_t nn_splitk_floats(long M, int N, int K) {
   return sp > 1 ? (size_t)sp * M * N : 0;
 }
 
+// the splits that conv_gemm takes, and K per split: 1 where the row tiles
+// fill the GPU or the scratch does not hold the partials
+int conv_splits(long M, int N, int K, const float *scratch, size_t scratch_floats, int *per) {
+  const int ksteps = (K + kGBK - 1) / kGBK;
+  int splits = choose_splits((M + kGBM - 1) / kGBM, ksteps, sm_count());
+  *per = ((ksteps + splits - 1) / splits) * kGBK;
+  splits = (K + *per - 1) / *per;
+  return splits > 1 && (!scratch || scratch_floats < (size_t)splits * M * N) ? 1 : splits;
+}
+
 // the conv GEMM of forward (sign +1) or dgrad (-1), split over K when the
 // row tiles alone cannot fill the GPU and the scratch allows
 template <class EPI_DIRECT>
@@ -1242,16 +1276,8 @@ cudaError_t conv_gemm(const void *a, const Vol &v, int ca, int ntaps, int sign, 
                       const void *mask, float *scratch, size_t scratch_floats, int *status,
                       cudaStream_t s) {
   const int K = ntaps * ca;
-  int sms = 148;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long mtiles = (M + kGBM - 1) / kGBM;
-  const int ksteps = (K + kGBK - 1) / kGBK;
-  int splits = choose_splits(mtiles, ksteps, sms);
-  const int per = ((ksteps + splits - 1) / splits) * kGBK;
-  splits = (K + per - 1) / per;
-  if (splits > 1 && (!scratch || scratch_floats < (size_t)splits * M * N)) splits = 1;
+  int per = 0;
+  const int splits = conv_splits(M, N, K, scratch, scratch_floats, &per);
   cudaError_t e = cudaErrorInvalidValue;
   dispatch_bn(N, [&](auto BNc) {
     constexpr int BN = decltype(BNc)::value;
@@ -1299,7 +1325,13 @@ cudaError_t nn_conv_dgrad(const void *dy, int B, int D, int H, int W, int cout, 
                           int cin, int ntaps, const void *mask, void *dx, float *scratch,
                           size_t scratch_floats, int *status, cudaStream_t s) {
   const long M = (long)B * D * H * W;
-  const int zt = g_gemm_only ? 0 : direct_planes(true, cout, cin, ntaps, B, D, H, W, sm_count());
+  // The direct kernel adds the taps and channels in the GEMM's order, so the
+  // gradients are the same bits; where the GEMM splits K (its FP32 sums then
+  // run in another order, and a BF16 result may round the other way) it stays.
+  int per = 0;
+  const int zt = g_gemm_only || conv_splits(M, cin, ntaps * cout, scratch, scratch_floats, &per) > 1
+                     ? 0
+                     : direct_planes(true, cout, cin, ntaps, B, D, H, W, sm_count());
   if (zt > 0 && al16(mask)) {
     const cudaError_t e = conv_direct<true>(zt, dy, B, D, H, W, cout, wt, nullptr, cin, 0, mask, dx,
                                             nullptr, status, s);
@@ -1337,7 +1369,7 @@ cudaError_t nn_conv_wgrad(const void *x, const void *dy, int B, int D, int H, in
   });
   if (e != cudaSuccess) return e;
   const long n = (long)cout * Mtot;
-  k_reduce_splits<<<(unsigned)((n + kReduceOuts - 1) / kReduceOuts), kEw, 0, s>>>(part, splits, n, dw);
+  sum_rows(part, splits, n, dw, s);
   return cudaGetLastError();
 }
 
@@ -1351,7 +1383,7 @@ cudaError_t nn_bias_grad(const void *dy, long M, int N, float *scratch, float *d
     k_bias_partial8<<<nb, kEw, 0, s>>>(static_cast<const bf16 *>(dy), M, N, scratch);
   else
     k_bias_partial<<<nb, kEw, 0, s>>>(static_cast<const bf16 *>(dy), M, N, scratch);
-  k_bias_final<<<N, kEw, 0, s>>>(scratch, nb, N, db);
+  sum_rows(scratch, nb, N, db, s);
   return cudaGetLastError();
 }
 

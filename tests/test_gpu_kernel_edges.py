@@ -12,7 +12,10 @@ oracle.
   order, more than fit the list, buckets left unsorted and sorted. Bit-exact.
 * The direct kernel's data gradient, with one, two and four planes a tile and
   with and without the ReLU mask: BF16 outputs to 1e-2 of max |ref|, the
-  bound of the GEMM path's test (one BF16 rounding is 2^-9).
+  bound of the GEMM path's test (one BF16 rounding is 2^-9), and the GEMM
+  path's own bits, its split K included.
+* The weight and bias gradients' FP32 sums over K splits and over rows, in
+  the order that the kernels state. Bit-exact.
 * Interpolation at the volume's borders, at positions just below zero (whose
   fraction is not a float), at integers, and beyond the range of the fast
   floor. Bit-exact.
@@ -104,6 +107,85 @@ def test_conv_dgrad_direct(grid, cin, cout, masked):
     assert rc == 0, _lib.lib().aw_last_error()
     got = host(dx.float()).reshape(want.shape)
     assert np.abs(got - want).max() <= 1e-2 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("grid", [(1, 32, 32, 32), (1, 28, 32, 24), (1, 40, 48, 32), (2, 8, 32, 40)])
+@pytest.mark.parametrize("cin,cout", [(16, 16), (48, 16), (16, 32), (32, 32)])
+@pytest.mark.parametrize("scratch", [True, False])
+def test_conv_dgrad_bits_do_not_depend_on_the_path(grid, cin, cout, scratch):
+    """With the scratch of aw_nn_conv3d_scratch_floats the GEMM splits K on the small grids (32^3: in three)
+    and not on the others; without it, nowhere."""
+    B, DD, H, W = grid
+    rng = np.random.default_rng(38)
+    dev = lambda a: torch.from_numpy(a).to(torch.bfloat16).cuda()  # noqa: E731
+    dy = dev(rng.normal(0, 1, grid + (cout,)).astype(np.float32))
+    wt = dev(rng.normal(0, 0.1, (cin, 27, cout)).astype(np.float32))
+    mask = dev(rng.normal(0, 1, grid + (cin,)).astype(np.float32))
+    L = _lib.lib()
+    n = int(L.aw_nn_conv3d_scratch_floats(*grid, cin, cout, 27)) if scratch else 0
+    sc = torch.zeros(max(n, 1), device="cuda")
+    got = []
+    for gemm in (0, 1):
+        dx = torch.zeros((B * DD * H * W, cin), dtype=torch.bfloat16, device="cuda")
+        L.aw_nn_set_gemm_only(gemm)
+        try:
+            rc = L.aw_nn_conv3d_dgrad(dy.data_ptr(), B, DD, H, W, cout, wt.data_ptr(), cin, 27, mask.data_ptr(),
+                                      dx.data_ptr(), sc.data_ptr() if n else None, n, None)
+        finally:
+            L.aw_nn_set_gemm_only(0)
+        assert rc == 0, L.aw_last_error()
+        got.append(dx)
+    assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("grid,splits", [((1, 8, 8, 8), 1), ((1, 8, 8, 8), 3), ((2, 8, 16, 64), 130),
+                                         ((1, 8, 48, 48), 288)])
+@pytest.mark.parametrize("cin,cout,taps", [(16, 16, 1), (32, 16, 27), (16, 48, 27)])
+def test_wgrad_splits_in_order(grid, splits, cin, cout, taps):
+    """dW is the sum of the splits' partial results, which the call leaves in its scratch, first to last."""
+    rng = np.random.default_rng(39)
+    B, DD, H, W = grid
+    x = torch.from_numpy(rng.normal(0, 1, grid + (cin,)).astype(np.float32)).to(torch.bfloat16).cuda()
+    dy = torch.from_numpy(rng.normal(0, 1, grid + (cout,)).astype(np.float32)).to(torch.bfloat16).cuda()
+    L = _lib.lib()
+    part = torch.zeros(int(L.aw_nn_wgrad_scratch_floats(cin, cout, taps, splits)), device="cuda")
+    dw = torch.zeros((cout, taps, cin), device="cuda")
+    rc = L.aw_nn_conv3d_wgrad(x.data_ptr(), dy.data_ptr(), B, DD, H, W, cin, cout, taps, splits, part.data_ptr(),
+                              dw.data_ptr(), None)
+    assert rc == 0, L.aw_last_error()
+    used = -(-B * DD * H * W // (-(-(-(-B * DD * H * W // splits)) // 64) * 64))  # splits of whole 64-voxel steps
+    want = np.zeros(dw.shape, np.float32)
+    for p in host(part).reshape(splits, cout, taps, cin)[:used]:
+        want = want + p
+    assert np.array_equal(host(dw), want)
+
+
+@pytest.mark.parametrize("cout", [1, 7, 16, 24, 32, 64, 128, 192, 256])
+@pytest.mark.parametrize("rows", [1, 511, 512, 1234, 512 * 130 + 3])
+def test_bias_sums_in_order(rows, cout):
+    """Blocks of 512 rows: every (256 / cout)-th row from each of the first ones, these sums first to last, then
+    the blocks first to last."""
+    rng = np.random.default_rng(40)
+    dy = torch.from_numpy(rng.normal(0, 1, (rows, cout)).astype(np.float32)).to(torch.bfloat16)
+    L = _lib.lib()
+    sc = torch.zeros(int(L.aw_nn_bias_scratch_floats(rows, cout)), device="cuda")
+    db = torch.zeros(cout, device="cuda")
+    d = dy.cuda()
+    assert L.aw_nn_bias_grad(d.data_ptr(), rows, cout, sc.data_ptr(), db.data_ptr(), None) == 0
+    blocks, groups = -(-rows // 512), 256 // cout
+    steps = -(-512 // groups)
+    y = np.zeros((blocks, 512, cout), np.float32)
+    y.reshape(-1, cout)[:rows] = dy.float().numpy()
+    y = np.concatenate([y, np.zeros((blocks, steps * groups - 512, cout), np.float32)], 1)
+    y = y.reshape(blocks, steps, groups, cout)  # adding a zero keeps a sum's bits
+
+    def in_order(a, axis):
+        t = np.zeros(np.delete(a.shape, axis), np.float32)
+        for k in range(a.shape[axis]):
+            t = t + np.take(a, k, axis)
+        return t
+    want = in_order(in_order(in_order(y, 1), 1), 0)
+    assert np.array_equal(host(db), want)
 
 
 def _edge_field(shape, rng):
