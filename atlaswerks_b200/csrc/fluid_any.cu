@@ -122,7 +122,10 @@ AW_D void with_solve_radix(int R, const F &f) {
 // butterflies in registers (over the pairs x[j] +- x[R-j], as dft<> does: 16
 // multiply-adds to a twiddle pair read, its index stepped by k modulo n), and
 // the block waits before any of the group's butterflies is written. kPrimeK:
-// 4 in the xy kernels, 3 in the z kernel, by their registers.
+// 4 in the slab kernels, 3 in the split and z kernels, by their registers. An
+// axis of at most 512 has at most 64 chunks of k there and 85 here, and a
+// block has the threads for them (128 and 256; a z block 64, and 256 from nz
+// = 389 on, the first with more chunks, whose tile lets two share an SM).
 template <int SIGN, int kPrimeK, class At>
 AW_D void prime_stage(float2 *S, const float2 *tw, const AnyStage &st, int n, int nlines,
                       const IdxDiv &byLines, const At &at) {
@@ -133,8 +136,11 @@ AW_D void prime_stage(float2 *S, const float2 *tw, const AnyStage &st, int n, in
   const int k0 = 1 + ch * kPrimeK;
   for (int base = 0; base < half; base += G) {
     const bool on = base + g < half && ch < nch;
-    // the two butterflies; an odd total's last pair is the same one twice
-    const int bf[2] = {base + g, min(base + g + half, total - 1)};
+    // Two butterflies, each of the stage's belonging to one thread of every
+    // chunk: groups are not parted by a barrier, so a butterfly that another
+    // group has too would be read after it was written. The thread of an odd
+    // total's middle one takes it twice.
+    const int bf[2] = {base + g, base + g + half < total ? base + g + half : base + g};
     float2 a[2][kPrimeK], b[2][kPrimeK], s[2];
     int w0[2], js[2], line[2];
     if (on) {

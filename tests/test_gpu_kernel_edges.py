@@ -65,6 +65,29 @@ def test_fluid_operator_any_axis(oracle, shape, inverse):
     assert not op.TimedOut()
 
 
+@pytest.mark.parametrize("shape,pairs", [
+    ((120, 45, 181), 0), ((120, 154, 155), 0), ((220, 167, 98), 0), ((120, 145, 153), 0), ((280, 81, 205), 0),
+    ((3, 245, 257), 16), ((5, 241, 271), 22), ((3, 331, 259), 0)])
+@pytest.mark.parametrize("inverse", [True, False])
+def test_fluid_prime_stage_leaves_one_over(oracle, shape, pairs, inverse):
+    """A prime above the register radices over an odd number of butterflies, the last of which falls into a group
+    of threads of its own: 385 in groups of 96, 49 in 12, 205 in 51, 23 in 11; on split grids the last batch's 11
+    or 11 lines of `pairs`."""
+    rng = np.random.default_rng(41)
+    sp = (1.0, 1.3, 0.8)
+    f = rng.normal(0, 1, (3,) + shape).astype(np.float32)
+    want = oracle.fluid_f64(f, sp, inverse=inverse)
+    op = DiffOperB200()
+    op.SetSize(shape[::-1], sp, DiffOperParam())
+    if pairs:
+        _lib.check(_lib.lib().aw_fluid_set_shapes(op._h, pairs, 16, 8))
+    v = cu(f)
+    (op.ApplyInverseOperator if inverse else op.ApplyOperator)(v)
+    err = np.abs(host(v).astype(np.float64) - want).max() / np.abs(want).max()
+    assert err <= 1e-5, err
+    assert not op.TimedOut()
+
+
 @pytest.mark.parametrize("shape", [(12, 11, 10), (9, 17, 131), (20, 18, 16)])
 @pytest.mark.parametrize("scale", [1.0, 0.85, 0.7, 0.55, 0.42, 0.3])
 @pytest.mark.parametrize("jitter", [0.0, 0.3])
