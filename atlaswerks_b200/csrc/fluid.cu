@@ -132,19 +132,26 @@ cudaError_t set_smem(const void *kernel, size_t bytes) {
   return e;
 }
 
-// Launch shapes of the any-size path. P row pairs and Q columns per CTA
-// (split grids; a slab that fits one CTA is its own batch), K columns per
-// z-pass CTA, taken up to a power of two between 8 and 32 whose tile fits.
+// what a block's dynamic shared memory may take: the kernels' barrier lies
+// before it, on 128 bytes with the alignment
+size_t any_smem_limit(int device) {
+  int maxsm = 0;
+  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  return (size_t)std::max(0, maxsm - 128);
+}
+
+// Launch shapes of the any-size path, into a. P row pairs and Q columns per
+// CTA (split grids; a slab that fits one CTA is its own batch), K columns per
+// z-pass CTA, taken up to a power of two between 8 and 32.
 // Threads: the xy kernels' registers allow 768 threads on an SM, the z
 // kernel's 1024: these are shared out over the CTAs that an SM gets, by
 // its shared memory and by the grid.
-void any_shapes(FluidPlan *p, int P, int Q, int K, size_t maxsm) {
-  p->pairs_per_batch = P;
-  p->cols_per_batch = Q;
-  p->zcols_per_cta = K;
-  AnyPlan &a = *p->any;
+// False: a kernel's shared memory would exceed maxsm. A slab in one CTA and a
+// z tile of 16 columns of 512 always fit (fluid_plan_create splits the
+// others); 32 columns do up to nz = 293.
+bool any_shapes(const FluidPlan &p, AnyPlan *a, int P, int Q, int K, size_t maxsm) {
   int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device);
   auto threads = [&](size_t smem, long ctas, int budget, int lo, int hi) {
     const long by_smem = std::max<long>(1, (long)((227u * 1024u) / (smem + 1024)));
     const long per_sm = std::max<long>(1, std::min<long>(by_smem, (ctas + sms - 1) / sms));
@@ -152,26 +159,17 @@ void any_shapes(FluidPlan *p, int P, int Q, int K, size_t maxsm) {
   };
   int q = 8;
   while (q < K && q < 32) q *= 2;
-  any_set_z(&a, q);
-  while (q > 8 && a.smem_z > maxsm) any_set_z(&a, q /= 2);
-  a.threads_z = threads(a.smem_z, (a.z.pcols + q - 1) / q, 1024, 64, 256);
-  a.smem_xy = any_smem_xy(a.xy);
-  a.threads_xy = threads(a.smem_xy, 3L * p->d.nz, 768, 128, 768);
-  any_set_split(&a, P, Q, maxsm);
+  any_set_z(a, q);
+  a->threads_z = threads(a->smem_z, (a->z.pcols + q - 1) / q, 1024, 64, 256);
+  a->smem_xy = any_smem_xy(a->xy);
+  a->threads_xy = threads(a->smem_xy, 3L * p.d.nz, 768, 128, 768);
+  any_set_split(a, P, Q, maxsm);
+  const bool xy = p.split ? a->smem_x <= maxsm && any_smem_y(a->xy, Q) <= maxsm : a->smem_xy <= maxsm;
+  return xy && a->smem_z <= maxsm;
 }
 
-// whether the shapes are within bounds: two complex buffers of each batch
-// in shared memory, next to the slab unless the grid is split
-bool any_fits(const FluidPlan &p, int P, int Q, int K, size_t maxsm) {
-  const size_t nx = p.d.nx, ny = p.d.ny, nz = p.d.nz, c = sizeof(float2);
-  const size_t x = 2 * c * P * nx, y = 2 * c * Q * ny;
-  const bool xy = p.split ? x <= maxsm && y <= maxsm
-                          : c * ny * p.nxh + std::max(x, y) <= maxsm;
-  return xy && 6 * c * K * nz <= maxsm;
-}
-
-cudaError_t any_configure(const FluidPlan &p) {
-  for (const auto &k : any_kernels(*p.any, p.split)) {
+cudaError_t any_configure(const AnyPlan &a, bool split) {
+  for (const auto &k : any_kernels(a, split)) {
     const cudaError_t e = set_smem(k.first, k.second);
     if (e != cudaSuccess) return e;
   }
@@ -236,11 +234,15 @@ cudaError_t fluid_set_shapes(FluidPlan *p, int P, int Q, int K) {
     return cudaSuccess;
   }
   if (P < 1 || P > npairs || Q < 1 || Q > p->nxh || K < 1 || K > 64) return cudaErrorInvalidValue;
-  int maxsm = 0;
-  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device);
-  if (!any_fits(*p, P, Q, K, (size_t)maxsm)) return cudaErrorInvalidValue;
-  any_shapes(p, P, Q, K, (size_t)maxsm);
-  return any_configure(*p);
+  AnyPlan a = *p->any;  // a rejected shape leaves the plan as it is
+  if (!any_shapes(*p, &a, P, Q, K, any_smem_limit(p->device))) return cudaErrorInvalidValue;
+  const cudaError_t e = any_configure(a, p->split);
+  if (e != cudaSuccess) return e;
+  *p->any = a;
+  p->pairs_per_batch = P;
+  p->cols_per_batch = Q;
+  p->zcols_per_cta = K;
+  return cudaSuccess;
 }
 
 // The any-size path's autotuner: on split grids every combination of half,
@@ -281,6 +283,7 @@ cudaError_t fluid_autotune(FluidPlan *p, cudaStream_t s) {
     return r;
   };
   float *c[3] = {f, f + n, f + 2 * n};
+  // the shapes that the plan holds stand unless a candidate beats them
   const int P0 = p->pairs_per_batch, Q0 = p->cols_per_batch, K0 = p->zcols_per_cta;
   int bestP = P0, bestQ = Q0, bestK = K0;
   float best = 1e30f;
@@ -354,14 +357,17 @@ int fluid_plan_create(FluidPlan *p, int nx, int ny, int nz, double spx, double s
     if (!p->any) return 3;
     if (!any_plan(p->any, &tab, p->d, p->sp, alpha, beta, gamma, false)) return 1;
     // a slab whose half spectrum does not fit one CTA: the split x / y passes
-    if (any_smem_xy(p->any->xy) > (size_t)maxsm) {
+    const size_t limit = any_smem_limit(dev);
+    if (any_smem_xy(p->any->xy) > limit) {
       p->split = 1;
       if (!any_plan(p->any, &tab, p->d, p->sp, alpha, beta, gamma, true)) return 1;
     }
     const int npairs = (ny + 1) / 2;
-    any_shapes(p, std::max(1, std::min(npairs, (2048 + nx - 1) / nx)),
-               std::max(1, std::min(p->nxh, p->split ? 32 : (2048 + ny - 1) / ny)),
-               std::max(1, std::min(16, 3072 / (3 * nz))), (size_t)maxsm);
+    p->pairs_per_batch = std::max(1, std::min(npairs, (2048 + nx - 1) / nx));
+    p->cols_per_batch = std::max(1, std::min(p->nxh, p->split ? 32 : (2048 + ny - 1) / ny));
+    p->zcols_per_cta = std::max(1, std::min(16, 3072 / (3 * nz)));
+    if (!any_shapes(*p, p->any, p->pairs_per_batch, p->cols_per_batch, p->zcols_per_cta, limit))
+      return 2;
   }
   const size_t spec_elems = p->fast ? 3 * (size_t)nz * ny * p->nxh
                                     : 3 * (size_t)nz * (size_t)p->any->xy.pcols;
@@ -388,7 +394,7 @@ int fluid_plan_create(FluidPlan *p, int nx, int ny, int nz, double spx, double s
   p->az.tw = p->tw + nx + ny;
   if (p->any) {
     if (!upload_any(p, tab)) return 3;
-    if (any_configure(*p) != cudaSuccess) return 4;
+    if (any_configure(*p->any, p->split) != cudaSuccess) return 4;
   }
   if (p->fast) p->fast_tma = encode_spec_map(p);
   if (p->fast && fast_configure(*p) != cudaSuccess) return 4;

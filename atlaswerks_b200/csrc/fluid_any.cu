@@ -1038,6 +1038,9 @@ void any_set_z(AnyPlan *p, int q) {
   p->smem_z = sizeof(float2) * (3 * (size_t)p->z.d.nz * q + p->z.d.nz) + sizeof(float4) * p->z.d.nz;
 }
 
+// shared memory of the split path's y pass with Q columns per block
+size_t any_smem_y(const AnyXY &a, int Q) { return sizeof(float2) * ((size_t)a.d.ny * Q + a.d.ny); }
+
 // the split path's row pairs (rounded up to even: a batch starts on 16
 // bytes) and columns (up to a power of two of at most 64 whose tile fits)
 // per block
@@ -1047,12 +1050,11 @@ void any_set_split(AnyPlan *p, int P, int Q, size_t maxsm) {
   a.byP = make_idxdiv((uint32_t)a.P);
   const int last = a.H - (a.H - 1) / a.P * a.P;
   a.byLast = make_idxdiv((uint32_t)last);
-  auto tile = [&](int q) { return sizeof(float2) * ((size_t)a.d.ny * q + a.d.ny); };
   a.Q = 1;
-  while (a.Q < Q && a.Q < 64 && tile(2 * a.Q) <= maxsm) a.Q *= 2;
+  while (a.Q < Q && a.Q < 64 && any_smem_y(a, 2 * a.Q) <= maxsm) a.Q *= 2;
   a.byQ = make_idxdiv((uint32_t)a.Q);
   p->smem_x = sizeof(float2) * ((((size_t)a.P * a.pitch + 1) & ~(size_t)1) + a.x.n);
-  p->smem_y = tile(a.Q);
+  p->smem_y = any_smem_y(a, a.Q);
   p->threads_y = a.Q >= 32 ? 512 : 256;
 }
 

@@ -103,6 +103,7 @@ struct AnyTables {
 bool any_plan(AnyPlan *p, AnyTables *t, const Dims &d, const Spacing &sp, float alpha, float beta,
               float gamma, bool split);
 size_t any_smem_xy(const AnyXY &a);
+size_t any_smem_y(const AnyXY &a, int Q);
 void any_set_z(AnyPlan *p, int q);
 void any_set_split(AnyPlan *p, int P, int Q, size_t maxsm);
 // the kernels of a plan and the shared memory each needs

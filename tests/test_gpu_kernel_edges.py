@@ -88,6 +88,41 @@ def test_fluid_prime_stage_leaves_one_over(oracle, shape, pairs, inverse):
     assert not op.TimedOut()
 
 
+# Slabs that fit one block without room for two more buffers of a batch, the largest that do (120 x 470 and
+# 312 x 182 would but for the block's barrier), and larger ones.
+@pytest.mark.parametrize("shape", [(3, 224, 224), (2, 220, 240), (3, 240, 208), (2, 200, 256), (2, 100, 512),
+                                   (2, 470, 120), (3, 182, 312), (2, 469, 119), (2, 472, 120), (2, 184, 312)])
+@pytest.mark.parametrize("inverse", [True, False])
+def test_fluid_slabs_at_the_limit_of_one_block(oracle, shape, inverse):
+    rng = np.random.default_rng(42)
+    sp = (1.0, 1.3, 0.8)
+    f = rng.normal(0, 1, (3,) + shape).astype(np.float32)
+    want = oracle.fluid_f64(f, sp, inverse=inverse)
+    op = DiffOperB200()
+    op.SetSize(shape[::-1], sp, DiffOperParam())
+    v = cu(f)
+    (op.ApplyInverseOperator if inverse else op.ApplyOperator)(v)
+    err = np.abs(host(v).astype(np.float64) - want).max() / np.abs(want).max()
+    assert err <= 1e-5, err
+    assert not op.TimedOut()
+
+
+@pytest.mark.parametrize("nz,fits", [(152, 1), (293, 1), (294, 0), (512, 0)])
+def test_fluid_z_tile_of_32_columns(oracle, nz, fits):
+    """Taken wherever its shared memory is there; a refused shape leaves the plan as it was."""
+    rng = np.random.default_rng(43)
+    f = rng.normal(0, 1, (3, nz, 5, 36)).astype(np.float32)
+    op = DiffOperB200()
+    op.SetSize((36, 5, nz), (1.0, 1.0, 1.0), DiffOperParam())
+    L = _lib.lib()
+    _lib.check(L.aw_fluid_set_shapes(op._h, 1, 1, 8))
+    want = host(op.ApplyInverseOperator(cu(f))).copy()
+    assert (L.aw_fluid_set_shapes(op._h, 1, 1, 32) == 0) == bool(fits)
+    assert np.array_equal(host(op.ApplyInverseOperator(cu(f))), want)
+    assert L.aw_fluid_set_shapes(op._h, 1, 1, 16) == 0
+    assert np.array_equal(host(op.ApplyInverseOperator(cu(f))), want)
+
+
 @pytest.mark.parametrize("shape", [(12, 11, 10), (9, 17, 131), (20, 18, 16)])
 @pytest.mark.parametrize("scale", [1.0, 0.85, 0.7, 0.55, 0.42, 0.3])
 @pytest.mark.parametrize("jitter", [0.0, 0.3])
