@@ -123,6 +123,23 @@ def test_fluid_z_tile_of_32_columns(oracle, nz, fits):
     assert np.array_equal(host(op.ApplyInverseOperator(cu(f))), want)
 
 
+@pytest.mark.parametrize("shape", [(12, 11, 10), (7, 18, 30), (16, 32, 16)])
+@pytest.mark.parametrize("k", [70, -70])
+def test_fluid_parameters_scale(shape, k):
+    """alpha, beta and gamma times a power of two scale every wavenumber's matrix by it, exactly: so does the
+    result, up to diagonal terms whose squares are no floats."""
+    rng = np.random.default_rng(44)
+    f = rng.normal(0, 1, (3,) + shape).astype(np.float32)
+    out = []
+    for s in (1.0, 2.0 ** k):
+        op = DiffOperB200()
+        op.SetSize(shape[::-1], (1.0, 1.3, 0.8), DiffOperParam(0.01 * s, 0.01 * s, 0.001 * s))
+        out.append((host(op.ApplyInverseOperator(cu(f))).copy(), host(op.ApplyOperator(cu(f))).copy()))
+    assert np.isfinite(out[1][0]).all() and np.isfinite(out[1][1]).all()
+    assert np.array_equal(out[1][0] * np.float32(2.0 ** k), out[0][0])
+    assert np.array_equal(out[1][1] * np.float32(2.0 ** -k), out[0][1])
+
+
 @pytest.mark.parametrize("shape", [(12, 11, 10), (9, 17, 131), (20, 18, 16)])
 @pytest.mark.parametrize("scale", [1.0, 0.85, 0.7, 0.55, 0.42, 0.3])
 @pytest.mark.parametrize("jitter", [0.0, 0.3])
