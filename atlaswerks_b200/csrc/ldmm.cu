@@ -1134,7 +1134,7 @@ cudaError_t ldmm_velshoot_iterate(LdmmCtx *c, const float *I0, const float *I1, 
 int ldmm_adshoot_prepare(LdmmCtx *c) {
   if (c->adV) return 0;
   const size_t n = (size_t)c->d.n(), T = (size_t)c->T;
-  const size_t sort_bytes = (splat_scratch_bytes(c->d) + 255) & ~size_t(255);
+  const size_t sort_bytes = (splat_scratch_bytes(c->d, false) + 255) & ~size_t(255);
   if (c->T + 1 > kMaxAdSorts) return 3;
   if (cudaMalloc(&c->adV, sizeof(float) * T * 3 * n) != cudaSuccess ||
       cudaMalloc(&c->adP, sizeof(float) * 2 * (T + 1) * 3 * n) != cudaSuccess ||
@@ -1149,8 +1149,10 @@ int ldmm_adshoot_prepare(LdmmCtx *c) {
     c->adSortMem = nullptr;
     return 3;
   }
-  for (size_t k = 0; k <= T; ++k)
-    splat_work_bind(&c->adSort[k], c->d, static_cast<char *>(c->adSortMem) + k * sort_bytes);
+  for (size_t k = 0; k <= T; ++k) {
+    splat_work_bind(&c->adSort[k], c->d, static_cast<char *>(c->adSortMem) + k * sort_bytes, false);
+    c->adSort[k].prod = c->sw.prod;  // rewritten by every gather, all on one stream
+  }
   return 0;
 }
 

@@ -44,7 +44,7 @@ struct LdmmCtx {
   float *adA;       // T x N: alpha_t = splat(alpha0, phi0T_t), t = 1 .. T
   float *adI;       // 6N: alphaHat, IHat, alphaTilde, ITilde and two scratch images
   double *venergy;  // vector-energy history ring, indexed like energy
-  void *adSortMem;  // T + 1 splat scratch sets
+  void *adSortMem;  // T + 1 splat scratch sets (their products in sw's)
   SplatWork adSort[kMaxAdSorts];  // the sorts by phi0T_t (t = 1..T) and by phiT0_T (slot 0)
 };
 

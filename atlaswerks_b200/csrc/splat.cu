@@ -625,6 +625,10 @@ void splat_work_bind(SplatWork *w, const Dims &d, void *scratch, bool products) 
   w->blocksums = reinterpret_cast<int *>(p);
   p += align256(sizeof(int) * w->nblocks);
   w->prod = products ? reinterpret_cast<float *>(p) : nullptr;
+  int dev = 0;
+  w->sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    cudaDeviceGetAttribute(&w->sms, cudaDevAttrMultiProcessorCount, dev);
 }
 
 cudaError_t splat_sort(const SplatWork &w, const float *hx, const float *hy, const float *hz,
@@ -656,7 +660,7 @@ cudaError_t splat_gather(const SplatWork &w, const float *img, const float *hx, 
                      hz, w.prod, w.offsets, w.order, w.cursor, out, bg};
   const unsigned grid = (unsigned)((d.n() + kGatherThreads - 1) / kGatherThreads);
   // seven blocks an SM, or one thread per destination
-  const unsigned queued = (unsigned)std::min<long>((d.n() + kQueuedThreads - 1) / kQueuedThreads, 7 * 148);
+  const unsigned queued = (unsigned)std::min<long>((d.n() + kQueuedThreads - 1) / kQueuedThreads, 7L * w.sms);
   if (w.prod) {
     launch_early(k_products, dim3((unsigned)((d.n() + 255) / 256)), 256, 0, s, w.order,
                  w.offsets + w.next, d.n(), img, hx, hy, hz, w.prod);

@@ -29,6 +29,7 @@ struct SplatWork {
   int *blocksums;   // scan partials
   int nblocks;
   float *prod;      // 8n or null: per corner, weight times value of the source at each position of order
+  int sms;          // multiprocessors of the device it was bound on
 };
 
 // bytes of device scratch one splat of grid d needs; products: room for the
@@ -43,7 +44,9 @@ cudaError_t splat(const SplatWork &w, const float *img, const float *hx, const f
                   const float *hz, float *out, float bg, cudaStream_t s);
 // the two halves of splat(): the bucket sort of the sources by h, kept in w,
 // and the ordered per-destination sums of img, which any number of images
-// splatted by the same h can share
+// splatted by the same h can share. A gather keeps the sort, but writes w's
+// prod and its queue in cursor: the gathers of one w, and those of sorts that
+// share a prod, are ordered on one stream.
 cudaError_t splat_sort(const SplatWork &w, const float *hx, const float *hy, const float *hz,
                        cudaStream_t s);
 cudaError_t splat_gather(const SplatWork &w, const float *img, const float *hx, const float *hy,

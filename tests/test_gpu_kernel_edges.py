@@ -28,6 +28,8 @@ torch = pytest.importorskip("torch")
 from atlaswerks_b200 import _lib  # noqa: E402
 from atlaswerks_b200 import device as D  # noqa: E402
 from atlaswerks_b200.greedy import DiffOperB200, DiffOperParam  # noqa: E402
+from atlaswerks_b200.ldmm import LDMMIteratorParam  # noqa: E402
+from atlaswerks_b200.shooting import LDMMAdShootingIteratorB200, LDMMShootingDefDataB200  # noqa: E402
 from oracle import identity  # noqa: E402
 from oracle import nn_oracle as O  # noqa: E402
 
@@ -162,6 +164,25 @@ def test_splat_scan_sizes(oracle, shape):
     img = rng.normal(0, 1, shape).astype(np.float32)
     h = (identity(shape) + rng.normal(0, 0.4, (3,) + shape)).astype(np.float32)
     assert np.array_equal(host(D.splat(cu(img), cu(h), 0.0)), oracle.splat(img, h, 0.0))
+
+
+def test_adjoint_shooting_memory():
+    """The T + 1 kept sorts share one buffer of products: a handle at 80 x 96 x 112 with T = 5 stays below the
+    fields' and the sorts' own memory plus one such buffer, which T + 2 of them would exceed by 100 MB."""
+    nz, ny, nx, T = 80, 96, 112, 5
+    n, cells = nz * ny * nx, (nz + 1) * (ny + 1) * (nx + 1)
+    z = torch.zeros((nz, ny, nx), device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    it = LDMMAdShootingIteratorB200((nx, ny, nz), n_time_steps=T)
+    it.SetScaleLevel((nx, ny, nz), (1.0, 1.0, 1.0), LDMMIteratorParam(DiffOperParam(), 1.0, 0.01, False))
+    data = LDMMShootingDefDataB200(z, z, (1.0, 1.0, 1.0))
+    it.Iterate(data)
+    torch.cuda.synchronize()
+    used = before - torch.cuda.mem_get_info()[0]
+    floats = (T + 11 + 3 * 2) * n + (3 * T + 6 * (T + 1) + T + 6) * n  # the handle's fields, the iteration's, the data's
+    sorts = (T + 2) * (2 * cells + n)
+    assert used <= 4 * (floats + sorts + 8 * n) + (64 << 20), used / 2 ** 20
 
 
 @pytest.mark.parametrize("grid", [(1, 8, 32, 16), (2, 6, 32, 24), (1, 3, 32, 16), (1, 32, 64, 64)])
