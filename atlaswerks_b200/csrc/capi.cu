@@ -395,6 +395,7 @@ int aw_greedy_set_fused_update(aw_greedy_t g, int on) {
   if (!g) return fail("aw_greedy_set_fused_update: null handle");
   AW_CUDA(cudaDeviceSynchronize(), "aw_greedy_set_fused_update (pending work)");
   g->ctx.no_fused_update = on ? 0 : 1;
+  g->ctx.always_fuse_update = on && on != 1;
   for (auto &kv : g->graphs) cudaGraphExecDestroy(kv.second);
   g->graphs.clear();  // captured iterations hold the other inverse/update kernels
   return 0;

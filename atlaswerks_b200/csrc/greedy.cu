@@ -15,8 +15,8 @@
 // GreedyWarp.txx:99), a max|v| reduction and eps = MaxPert / max|v| computed
 // on the device (GreedyIteratorCPU.cxx:125-131). On small grids of the
 // register-FFT path, iterations without a step update or an inverse field
-// run 5 and 6 as one kernel (k_xy_inv_compose, fluid_fast.cu; the limit and
-// its reason are at kFuseVoxels): five launches.
+// run 5 and 6 as one kernel (k_xy_inv_compose, fluid_fast.cu) where that is
+// faster (fused_update_pays): five launches.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -461,12 +461,19 @@ void tune_update_tile(GreedyCtx *g) {
   g_tile[key] = pick;
 }
 
-// Up to here the inverse transform and the update run as one kernel (v never
-// leaves the chip, one launch less); beyond, the update on its own, with h
-// staged by TMA and its own registers and occupancy, is faster: 32^3 6.1
-// against 6.5 us plus a launch, 64^3 12.7 against 11.8, 128^3 51.7 against
-// 47.2, 128 x 128 x 256 (256 wide: one slab per SM) 184 against 94.
-constexpr long kFuseVoxels = 64L * 64 * 63;
+// Whether the inverse transform and the update run as one kernel (v never
+// leaves the chip, one launch less) or the update on its own, with its own
+// registers and occupancy. Microseconds an iteration, fused against separate:
+// * nx >= 64, where the separate update stages h by TMA: 64 x 32 x 32 19.2 /
+//   20.2, 128 x 32 x 32 27.4 / 25.2, 64^3 31.4 / 29.5, 128^3 117.8 / 111.6,
+//   256 x 128 x 128 354 / 261.
+// * nx = 16 and 32, where it gathers from global memory: 32^3 17.2 / 16.2, 16 x
+//   64 x 64 20.5 / 23.4, 32 x 64 x 128 32.6 / 35.6 (32 x 128 x 64 36.8 /
+//   36.2), 16 x 256 x 256 109 / 136.
+constexpr long kFuseVoxels = 65536;
+bool fused_update_pays(const Dims &d) {
+  return d.nx >= 64 ? d.n() <= kFuseVoxels : d.n() >= kFuseVoxels;
+}
 
 // the update on its own: h staged in shared memory where it can be, else
 // gathered from global memory. fast: the float-tree interpolation, which
@@ -602,7 +609,7 @@ cudaError_t greedy_stage(GreedyCtx *g, int stage, const float *I0, const float *
     case kStageInvCompose: {
       // grids the fused kernel does not take, or takes more slowly, run the
       // two stages it replaces
-      if (!g->plan.fast || d.n() > kFuseVoxels) {
+      if (!g->plan.fast || !(g->always_fuse_update || fused_update_pays(d))) {
         AW_TRY(greedy_stage(g, kStageXYInverse, I0, I1, h, h_out, hinv, hinv_out, auto_reduce,
                             solve_inverse, s));
         return update_stage(g, h, h_out, nullptr, nullptr, g->plan.fast && g->fast_interp, s);
@@ -621,8 +628,8 @@ cudaError_t greedy_stage(GreedyCtx *g, int stage, const float *I0, const float *
 // writers of the step it may reduce (AutoStepReduce).
 //
 // Without a step-size update or an inverse field, on the register-FFT path
-// up to kFuseVoxels, the inverse transform and the update are one kernel (kStageInvCompose):
-// v = K f stays in shared memory. The step update needs max |v| over the
+// where fused_update_pays, the inverse transform and the update are one kernel
+// (kStageInvCompose): v = K f stays in shared memory. The step update needs max |v| over the
 // whole field before any voxel moves, and the inverse field gathers v at
 // h^-1(x) anywhere in the volume, so those iterations store v.
 cudaError_t greedy_iterate(GreedyCtx *g, const float *I0, const float *I1, const float *const h[3],

@@ -33,6 +33,7 @@ struct GreedyCtx {
   void *hmaps;      // host cache of the h planes' tensor maps (greedy.cu)
   int no_staged_update;  // 1: the update gathers h from global memory only
   int no_fused_update;   // 1: v goes to HBM and a separate kernel updates h
+  int always_fuse_update;  // 1: one kernel for both wherever it can be
   int fast_interp;       // 1: float-tree interpolation in force-prep and the fused update
   int utile;             // tile shape of the staged update (greedy.cu)
 };

@@ -210,18 +210,19 @@ int aw_greedy_set_auto_step_reduce(aw_greedy_t g, int on);
  * ny >= 10, nz >= 6, no inverse field); 0: every gather from global memory.
  * Both give the same bits; the switch exists to compare them. */
 int aw_greedy_set_staged_update(aw_greedy_t g, int on);
-/* on = 1 (default): an iteration without a step-size update or an inverse
- * field, on a grid of power-of-two axes smaller than 64^3 voxels, runs the
- * inverse transform and the update h' = h(x + eps v/sp) as one kernel, so
- * v = K f never goes to HBM (the stages GreedyIteratorGPU::Iterate runs as
- * cplFFT inverse and composeHV, Greedy/GreedyIteratorGPU.cxx:120-134); 0,
- * and on larger grids, where it is faster: v is stored and the update is a
- * kernel of its own. Both give the same bits. */
+/* on = 2: an iteration without a step-size update or an inverse field, on a
+ * grid of power-of-two axes in [16, 256], runs the inverse transform and the
+ * update h' = h(x + eps v/sp) as one kernel, so v = K f never goes to HBM (the
+ * stages GreedyIteratorGPU::Iterate runs as cplFFT inverse and composeHV,
+ * Greedy/GreedyIteratorGPU.cxx:120-134); 1 (default): where that was measured
+ * faster, nx >= 64 and up to 65536 voxels, or nx < 64 and from 65536 on;
+ * 0: v is stored and the update is a kernel of its own everywhere. All give
+ * the same bits. */
 int aw_greedy_set_fused_update(aw_greedy_t g, int on);
 /* on = 1: I0(h) in the force preparation and h(x + eps v/sp) in the update
- * of an iteration that set_fused_update covers (power-of-two axes of any
- * size, no step update, no inverse field) interpolate with float fused multiply-adds instead of the
- * reference's double weights and sums: a few float ulps from the
+ * of an iteration that set_fused_update (1 or 2) covers, by either kernel
+ * (power-of-two axes in [16, 256], no step update, no inverse field),
+ * interpolate with float fused multiply-adds instead of the reference's double weights and sums: a few float ulps from the
  * bit-exact results (I0(h) within 1e-6 of it for images in [0, 1]); 0
  * (default): bit-exact with the reference CPU's interpolation. */
 int aw_greedy_set_fast_interpolation(aw_greedy_t g, int on);

@@ -27,9 +27,11 @@ torch = pytest.importorskip("torch")
 
 from atlaswerks_b200 import _lib  # noqa: E402
 from atlaswerks_b200 import device as D  # noqa: E402
-from atlaswerks_b200.greedy import DiffOperB200, DiffOperParam  # noqa: E402
+from atlaswerks_b200.greedy import (DiffOperB200, DiffOperParam, GreedyDeformationDataB200,  # noqa: E402
+                                    GreedyIteratorB200, GreedyIteratorParam)
 from atlaswerks_b200.ldmm import LDMMIteratorParam  # noqa: E402
 from atlaswerks_b200.shooting import LDMMAdShootingIteratorB200, LDMMShootingDefDataB200  # noqa: E402
+from atlaswerks_b200.synth import greedy_pair  # noqa: E402
 from oracle import identity  # noqa: E402
 from oracle import nn_oracle as O  # noqa: E402
 
@@ -168,7 +170,7 @@ def test_splat_scan_sizes(oracle, shape):
 
 def test_adjoint_shooting_memory():
     """The T + 1 kept sorts share one buffer of products: a handle at 80 x 96 x 112 with T = 5 stays below the
-    fields' and the sorts' own memory plus one such buffer, which T + 2 of them would exceed by 100 MB."""
+    fields' and the sorts' own memory plus one such buffer, which T + 2 of them would exceed by 90 MB."""
     nz, ny, nx, T = 80, 96, 112, 5
     n, cells = nz * ny * nx, (nz + 1) * (ny + 1) * (nx + 1)
     z = torch.zeros((nz, ny, nx), device="cuda")
@@ -282,6 +284,37 @@ def test_bias_sums_in_order(rows, cout):
         return t
     want = in_order(in_order(in_order(y, 1), 1), 0)
     assert np.array_equal(host(db), want)
+
+
+@pytest.mark.parametrize("shape,sp,max_pert", [((64, 64, 64), (1.0, 1.0, 1.0), 0.5),
+                                               ((128, 128, 128), (1.0, 1.0, 1.0), 0.5),
+                                               ((16, 32, 128), (2.0, 1.3, 0.8), 3.0),   # 65536: fused
+                                               ((32, 32, 128), (1.0, 1.3, 0.8), 0.5),   # the next: separate
+                                               ((32, 64, 32), (1.0, 1.0, 1.0), 2.0),    # 65536, narrow: fused
+                                               ((32, 32, 32), (1.0, 1.0, 1.0), 0.5),    # below: separate
+                                               ((16, 64, 256), (1.0, 1.0, 1.5), 3.0)])
+def test_fused_update_on_either_side_of_its_rule(shape, sp, max_pert):
+    """One kernel for the inverse transform and the update (2), two (0) and the rule's choice (1): the same bits,
+    with the float interpolation too where both run it."""
+    I0, I1 = greedy_pair(shape, seed=13)
+    L = _lib.lib()
+
+    def run(fused, fast):
+        it = GreedyIteratorB200(shape[::-1], spacing=sp)
+        it.SetScaleLevel(shape[::-1], sp, GreedyIteratorParam(DiffOperParam(0.01, 0.01, 0.001), max_pert))
+        _lib.check(L.aw_greedy_set_fused_update(it._h, fused))
+        it.SetFastInterpolation(fast)
+        d = GreedyDeformationDataB200(cu(I0), cu(I1), spacing=sp)
+        it.Run(d, 5, update_first=True)
+        return host(d.Def1To0()).copy(), it.Energies()
+    h, e = run(0, False)
+    assert np.abs(h - identity(shape)).max() > 0.1
+    for fused in (1, 2):
+        got = run(fused, False)
+        assert np.array_equal(got[0], h) and np.array_equal(got[1], e)
+    f1, f2 = run(1, True), run(2, True)
+    assert np.array_equal(f1[0], f2[0]) and np.array_equal(f1[1], f2[1])
+    assert not np.array_equal(f1[0], h)  # the float tree ran
 
 
 def _edge_field(shape, rng):
