@@ -119,12 +119,17 @@ __device__ __forceinline__ void cp_async_wait() {
 // voxel-index offset of each tap a second table, both made once per CTA in
 // shared memory. The L1 / shared-memory data pipe bounds these GEMMs (73 % of
 // its peak over the 96 -> 32 layer at 32^3, 90 % while its CTAs run, the
-// tensor pipe idle), so the copies pass L1 by and a warp's take 8 rows x 4
-// chunks at a time, 64 contiguous bytes a row. Against one row a thread
-// through L1: 96 -> 32 at 32^3 67.9 -> 64.4 us (the tensor work of it takes
-// 3.4), the 64-column layers at 16^3
-// 18.0 -> 14.4, the 128-column ones at 8^3 9.1 -> 8.9, 16 -> 16 with one tap
-// at 64^3 15.2 -> 16.0.
+// tensor pipe idle).
+// WIDE: the copies pass L1 by and a warp's take 8 rows x 4 chunks at a time,
+// 64 contiguous bytes a row. Else a thread takes one row, through L1, where
+// the taps of a short row (16 channels: 32 bytes) share their lines.
+// Microseconds a layer, a row a thread against WIDE: 16 -> 16 at 64^3 50 / 65,
+// 16 -> 32 at 32^3 25.4 / 27.0, 32 -> 32 there 33.6 / 35.7, 32 -> 64 50.0 /
+// 49.8, 64 -> 64 at 16^3 17.1 / 15.2, 128 -> 128 there 43 / 39, 192 -> 64 46 /
+// 33; with fewer than 64 columns 48 -> 16 at 16^3 10.0 / 10.6, 32^3 38.0 / 36.8,
+// 64^3 212 / 182, 96 -> 32 at 16^3 16.7 / 17.3, 24^3 38.1 / 38.4, 32^3 75 / 71.
+inline bool conv_wide(int C, int N, long M) { return C >= 48 && (N >= 64 || M >= 32768); }
+template <bool WIDE>
 struct LoadConvA {
   const bf16 *x;
   Vol v;
@@ -133,13 +138,14 @@ struct LoadConvA {
   FastDiv fc;
   static constexpr int kMN = 0;
   struct Ctx {
-    int m0;
-    const uint32_t *vmask;
+    int m0;                 // the tile's first row (WIDE), or the thread's row
+    uint32_t own;           // the thread's row's taps
+    const uint32_t *vmask;  // WIDE: those of all rows
     const int *toff;
   };
   AW_D Ctx init(long m0) const {
     __shared__ int s_toff[27];
-    __shared__ uint32_t s_vmask[kGBM];
+    __shared__ uint32_t s_vmask[WIDE ? kGBM : 1];
     if (threadIdx.x < ntaps) {
       int dz, dy, dx;
       tap_offset(threadIdx.x, ntaps, dz, dy, dx);
@@ -157,11 +163,27 @@ struct LoadConvA {
         if (zz >= 0 && zz < v.D && yy >= 0 && yy < v.H && xs >= 0 && xs < v.W) mask |= 1u << t;
       }
     }
-    s_vmask[threadIdx.x] = mask;
-    return Ctx{(int)m0, s_vmask, s_toff};  // the caller synchronises the CTA before the first issue()
+    if (WIDE) s_vmask[threadIdx.x] = mask;
+    return Ctx{WIDE ? (int)m0 : m, mask, s_vmask, s_toff};  // the caller synchronises the CTA before the first issue()
   }
   AW_D void issue(const Ctx &c, uint8_t *s, int k0, int kend) const {
     static_assert(kGThreads == 128 && kGBM == 128 && kGBK == 64, "copy layout");
+    if constexpr (!WIDE) {
+      int tap = (int)fc.div((uint32_t)k0);
+      int ci = k0 - tap * C;
+#pragma unroll
+      for (int j = 0; j < kGBK / 8; ++j) {
+        const bool ok = ((c.own >> tap) & 1u) && (k0 + 8 * j < kend);
+        const bf16 *src = ok ? x + (long)(c.m0 + c.toff[tap]) * C + ci : x;
+        cp_async16(s + kmajor_off(threadIdx.x, j, kGBM), src, ok);
+        ci += 8;
+        if (ci == C) {
+          ci = 0;
+          ++tap;
+        }
+      }
+      return;
+    }
     const int j0 = threadIdx.x & 3, r0 = threadIdx.x >> 2;
     uint32_t vm[4];
 #pragma unroll
@@ -1279,9 +1301,9 @@ cudaError_t conv_gemm(const void *a, const Vol &v, int ca, int ntaps, int sign, 
   int per = 0;
   const int splits = conv_splits(M, N, K, scratch, scratch_floats, &per);
   cudaError_t e = cudaErrorInvalidValue;
-  dispatch_bn(N, [&](auto BNc) {
+  auto run = [&](auto BNc, auto Wide) {
     constexpr int BN = decltype(BNc)::value;
-    LoadConvA la{static_cast<const bf16 *>(a), v, ca, ntaps, sign, (int)M, make_fastdiv(ca)};
+    LoadConvA<decltype(Wide)::value> la{static_cast<const bf16 *>(a), v, ca, ntaps, sign, (int)M, make_fastdiv(ca)};
     LoadRowsB<BN> lb{static_cast<const bf16 *>(b), K};
     if (splits > 1) {
       EpiPartial<BN> ep{scratch, M};
@@ -1299,6 +1321,12 @@ cudaError_t conv_gemm(const void *a, const Vol &v, int ca, int ntaps, int sign, 
       EpiMask<BN> ep{static_cast<const bf16 *>(mask), static_cast<bf16 *>(out), M};
       e = launch_gemm<BN>(la, lb, ep, M, K, 1, K, status, s);
     }
+  };
+  dispatch_bn(N, [&](auto BNc) {
+    if (conv_wide(ca, N, M))
+      run(BNc, std::true_type());
+    else
+      run(BNc, std::false_type());
   });
   return e;
 }

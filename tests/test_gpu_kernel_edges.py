@@ -236,6 +236,26 @@ def test_conv_dgrad_bits_do_not_depend_on_the_path(grid, cin, cout, scratch):
     assert torch.equal(got[0], got[1])
 
 
+@pytest.mark.parametrize("grid", [(1, 31, 32, 33), (1, 29, 36, 32), (1, 5, 7, 9)])  # 32736, 33408 and 315 rows
+@pytest.mark.parametrize("cin,cout,taps", [(48, 16, 27), (96, 32, 27), (32, 16, 27), (64, 64, 1), (48, 48, 1)])
+def test_conv_operand_loaders(grid, cin, cout, taps):
+    """Below 64 columns the GEMM's rows come 64 bytes of eight rows a warp from 48 channels and 32768 rows on, else
+    a row a thread: ragged last tiles on either side, to the bound of the GEMM's other tests."""
+    B, DD, H, W = grid
+    rng = np.random.default_rng(45)
+    x = O.bf16(rng.normal(0, 1, grid + (cin,)).astype(np.float32))
+    w = O.bf16(rng.normal(0, 0.1, (cout, taps, cin)).astype(np.float32))
+    b = rng.normal(0, 0.1, cout).astype(np.float32)
+    want = O.conv_fwd(x, w, b, relu=False)
+    xd, wd = (torch.from_numpy(a).to(torch.bfloat16).cuda() for a in (x, w))
+    bd = torch.from_numpy(b).cuda()
+    out = torch.zeros((B * DD * H * W, cout), device="cuda")
+    rc = _lib.lib().aw_nn_conv3d_fwd(xd.data_ptr(), B, DD, H, W, cin, wd.data_ptr(), bd.data_ptr(), cout, taps, 0,
+                                     None, out.data_ptr(), None, 0, None)
+    assert rc == 0, _lib.lib().aw_last_error()
+    assert np.abs(host(out).reshape(want.shape) - want).max() <= 1e-3 * np.abs(want).max()
+
+
 @pytest.mark.parametrize("grid,splits", [((1, 8, 8, 8), 1), ((1, 8, 8, 8), 3), ((2, 8, 16, 64), 130),
                                          ((1, 8, 48, 48), 288)])
 @pytest.mark.parametrize("cin,cout,taps", [(16, 16, 1), (32, 16, 27), (16, 48, 27)])
