@@ -542,22 +542,38 @@ int aw_greedy_profile(aw_greedy_t g, const float *I0, const float *I1, const flo
   AW_CUDA(cudaEventCreate(&e0), "aw_greedy_profile (event)");
   AW_CUDA(cudaEventCreate(&e1), "aw_greedy_profile (event)");
   int rc = 0;
+  auto run = [&](int stage) {
+    return aw::greedy_stage(&g->ctx, stage, I0, I1, h, o, inv ? hi : nullptr, inv ? hio : nullptr, 0,
+                            1, s);
+  };
+  // The spectrum of the iteration's velocity. A solve scales by 1 / (nx ny), so
+  // repeated ones take it to zero, where v and the step are no numbers and the
+  // update takes a third longer; an inverse transform of split slabs works in
+  // place. After the one, and before every launch of the other, it is formed
+  // again, outside the timed launches.
+  auto solved = [&]() {
+    const cudaError_t e = run(aw::kStageXYForward);
+    return e == cudaSuccess ? run(aw::kStageZSolve) : e;
+  };
   for (int stage = 0; stage < aw::kNumStages && rc == 0; ++stage) {
-    cudaError_t e = cudaEventRecord(e0, s);
-    for (int r = 0; r < reps && e == cudaSuccess; ++r)
-      e = aw::greedy_stage(&g->ctx, stage, I0, I1, h, o, inv ? hi : nullptr, inv ? hio : nullptr,
-                           0, (r & 1) ? 0 : 1, s);
-    if (e == cudaSuccess) e = cudaEventRecord(e1, s);
-    // the repetitions alternate K and L, which keeps the spectrum's scale; the
-    // stages that follow run on a solved one, the smooth velocity of an
-    // iteration (on the force itself the update takes a third longer)
-    if (e == cudaSuccess && stage == aw::kStageZSolve && !(reps & 1))
-      e = aw::greedy_stage(&g->ctx, stage, I0, I1, h, o, nullptr, nullptr, 0, 1, s);
-    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-    float ms = 0.f;
-    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+    const bool in_place = g->ctx.plan.split &&
+                          (stage == aw::kStageXYInverse || stage == aw::kStageInvCompose);
+    const int batches = in_place ? reps : 1;
+    cudaError_t e = cudaSuccess;
+    float total = 0.f;
+    for (int b = 0; b < batches && e == cudaSuccess; ++b) {
+      if (in_place) e = solved();
+      if (e == cudaSuccess) e = cudaEventRecord(e0, s);
+      for (int r = 0; r < reps / batches && e == cudaSuccess; ++r) e = run(stage);
+      if (e == cudaSuccess) e = cudaEventRecord(e1, s);
+      if (e == cudaSuccess && stage == aw::kStageZSolve) e = solved();
+      if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+      float ms = 0.f;
+      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+      total += ms;
+    }
     if (e != cudaSuccess) rc = cuda_fail(e, "aw_greedy_profile");
-    ms_out[stage] = ms / reps;
+    ms_out[stage] = total / reps;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);

@@ -254,11 +254,9 @@ int aw_greedy_run(aw_greedy_t g, const float *I0, const float *I1, float *hx, fl
  * 1 energy, 2 xy-forward FFT, 3 z-solve, 4 xy-inverse FFT, 5 max-norm,
  * 6 update, 7 xy-inverse FFT fused with the update, or stages 4 and 6 where
  * an iteration runs those) is launched `reps` times
- * back to back between CUDA events on `stream`, on the data of an iteration
- * (z-solve alternates K and L, the stages after it run on K f); ms_out[8]
- * receives the mean milliseconds per launch. Leaves h_out holding one
- * iteration's result (not on grids beyond one CTA's slab, whose inverse pass
- * works in place); records extra energies. Synchronises. */
+ * back to back between CUDA events on `stream`, on the data of an iteration;
+ * ms_out[8] receives the mean milliseconds per launch. Leaves h_out holding
+ * one iteration's result; records extra energies. Synchronises. */
 int aw_greedy_profile(aw_greedy_t g, const float *I0, const float *I1, const float *hx,
                       const float *hy, const float *hz, float *ox, float *oy, float *oz,
                       const float *hix, const float *hiy, const float *hiz, float *hiox,

@@ -337,11 +337,11 @@ def test_fused_update_on_either_side_of_its_rule(shape, sp, max_pert):
     assert not np.array_equal(f1[0], h)  # the float tree ran
 
 
-@pytest.mark.parametrize("shape", [(32, 32, 64), (24, 20, 28)])
-@pytest.mark.parametrize("reps", [1, 2, 3])
+@pytest.mark.parametrize("shape", [(32, 32, 64), (24, 20, 28), (6, 260, 250)])
+@pytest.mark.parametrize("reps", [1, 2, 25])
 def test_profile_leaves_one_iteration(shape, reps):
-    """The stages run on an iteration's own data: h_out is the iteration's result, bit for bit with one repetition,
-    and to the rounding of K L K against K with more (1e-6 of a voxel times the step's 0.5, bounded by 1e-4)."""
+    """The stages run on an iteration's own data however often each is repeated: h_out is the iteration's result,
+    bit for bit, on split slabs too."""
     import ctypes
     I0, I1 = (cu(a) for a in greedy_pair(shape, seed=13))
     it = GreedyIteratorB200(shape[::-1])
@@ -355,9 +355,7 @@ def test_profile_leaves_one_iteration(shape, reps):
     _lib.check(_lib.lib().aw_greedy_profile(it._h, I0.data_ptr(), I1.data_ptr(), *[t.data_ptr() for t in h],
                                             *[t.data_ptr() for t in ho], *z, *z, reps, None, ms))
     assert np.abs(want - identity(shape)).max() > 0.2
-    if reps == 1:
-        assert np.array_equal(host(ho), want)
-    assert np.abs(host(ho) - want).max() <= 1e-4
+    assert np.array_equal(host(ho), want)
 
 
 def _edge_field(shape, rng):
