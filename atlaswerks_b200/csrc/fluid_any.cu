@@ -8,7 +8,7 @@
 //   z solve      one block per Q consecutive places of a slab, all three
 //                components: the first radix is read from HBM straight into
 //                registers, the last one, the 3 x 3 solve and the inverse's
-//                first stay in registers (radices up to 10), and the
+//                first stay in registers (radices up to 5), and the
 //                inverse's last goes back to HBM from registers: the tile
 //                crosses shared memory four times in all for a length of two
 //                factors.
@@ -102,6 +102,7 @@ AW_D void with_even_radix(int R, const F &f) {
     AW_RADIX(16, kXYRadix)
   }
 }
+static_assert(kSolveRadix == 5, "the radices of the fused z step");
 template <class F>
 AW_D void with_solve_radix(int R, const F &f) {
   switch (R) {
@@ -109,11 +110,6 @@ AW_D void with_solve_radix(int R, const F &f) {
     AW_RADIX(3, kSolveRadix)
     AW_RADIX(4, kSolveRadix)
     AW_RADIX(5, kSolveRadix)
-    AW_RADIX(6, kSolveRadix)
-    AW_RADIX(7, kSolveRadix)
-    AW_RADIX(8, kSolveRadix)
-    AW_RADIX(9, kSolveRadix)
-    AW_RADIX(10, kSolveRadix)
   }
 }
 

@@ -191,7 +191,8 @@ class GreedyIteratorB200:
 
     def SetFastInterpolation(self, on: bool):
         """Float fused-multiply-add interpolation in the force preparation
-        and the fused update (a few float ulps from the bit-exact path)."""
+        and, on grids of power-of-two axes, in the update of iterations without
+        a step update or h^-1 (a few float ulps from the bit-exact path)."""
         check(_lib.lib().aw_greedy_set_fast_interpolation(self._h, int(on)))
 
     def SetAutoStepReduce(self, on: bool):
