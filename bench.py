@@ -19,7 +19,8 @@ per-rank device times.
 
 --impl reference times the reference's own CPU implementation
 (GreedyIteratorCPU, built from its sources into oracle/_ref) on the host
-cores, one 128^3 pair per thread.
+cores, one 128^3 pair per thread; without that build it prints an
+"unavailable" line.
 """
 from __future__ import annotations
 
@@ -174,36 +175,23 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return 0
-    from oracle import REF_SO, Oracle, Reference, identity
-    kind = "reference" if os.path.exists(REF_SO) else "port"
+    from oracle import REF_SO, Reference
+    if not os.path.exists(REF_SO):
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "the reference's CPU build (oracle/_ref/libawref.so) is absent: no reference "
+                          "source tree at build time"}))
+        return 0
     cores = max(1, min(os.cpu_count() or 1, 32))
     pairs = [make_pair(1000 + t) for t in range(cores)]
-    if kind == "reference":
-        ref = Reference()
-        handles = [None] * cores
+    ref = Reference()
+    handles = [None] * cores
 
-        def opener(t):
-            handles[t] = ref.greedy_open(*pairs[t], max_pert=MAX_PERT, alpha=ALPHA, beta=BETA,
-                                         gamma=GAMMA)
+    def opener(t):
+        handles[t] = ref.greedy_open(*pairs[t], max_pert=MAX_PERT, alpha=ALPHA, beta=BETA,
+                                     gamma=GAMMA)
 
-        def worker(t):
-            ref.greedy_iterate(handles[t], 1)
-    else:
-        o = Oracle()
-        state = [None] * cores
-
-        def opener(t):
-            I0, I1 = pairs[t]
-            h = identity(I0.shape)
-            _, st = o.greedy_iterate(I0, I1, h, None, max_pert=MAX_PERT, alpha=ALPHA, beta=BETA,
-                                     gamma=GAMMA, update_step=True)
-            state[t] = (h, st)
-
-        def worker(t):
-            I0, I1 = pairs[t]
-            h, st = state[t]
-            o.greedy_iterate(I0, I1, h, None, max_pert=MAX_PERT, alpha=ALPHA, beta=BETA,
-                             gamma=GAMMA, step=st)
+    def worker(t):
+        ref.greedy_iterate(handles[t], 1)
 
     def parallel(fn):
         th = [threading.Thread(target=fn, args=(t,)) for t in range(cores)]
@@ -220,9 +208,8 @@ def run_reference(args):
     for _ in range(args.steps):
         parallel(worker)
     dt = time.perf_counter() - t
-    if kind == "reference":
-        for h in handles:
-            ref.greedy_close(h)
+    for h in handles:
+        ref.greedy_close(h)
     value = args.steps * cores / dt
     line = {"metric": "128^3 fluid iters/s", "value": value, "unit": "iters/s",
             "impl": "reference", "n_gpus": int(os.environ.get("WORLD_SIZE", "1")),
@@ -236,7 +223,7 @@ def run_reference(args):
                                           f"the timed region)"}),
             "fft": "the reference's DiffOper over an FP64 FFTW-API shim: FFTW is not installed, "
                    "so single-precision FFTW would be faster than this arm",
-            "cpu_baseline": {"value": value, "unit": "iters/s", "cores": cores, "kind": kind,
+            "cpu_baseline": {"value": value, "unit": "iters/s", "cores": cores, "kind": "reference",
                              "sample": f"{args.steps} steps x {cores} threads x 1 steady-state "
                                        f"iteration of a {N}^3 pair (GreedyIteratorCPU; FFT = "
                                        f"FP64 shim, not FFTW)"},

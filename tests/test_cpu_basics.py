@@ -84,3 +84,20 @@ def test_static_splat_capacity_query():
     assert L.aw_splat_static_fits(89, 89, 89) == 0
     assert L.aw_splat_static_fits(0, 8, 8) == 0
     assert L.aw_splat_static_fits(400, 100, 1) == 1
+
+
+def test_reference_arm_without_the_reference_build():
+    """The benchmark's reference arm runs the reference's own code or says that it is not there; this project's
+    restatement does not stand in for it."""
+    import json
+    import subprocess
+    import sys
+    from oracle import REF_SO
+    if os.path.exists(REF_SO):
+        pytest.skip("the reference's CPU build is present")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "bench.py", "--impl", "reference", "--steps", "1", "--warmup", "3"], cwd=root,
+                       capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr
+    line = json.loads(r.stdout.strip().splitlines()[-1])
+    assert set(line) == {"impl", "unavailable"} and line["impl"] == "reference"
