@@ -395,6 +395,16 @@ def test_compose_at_the_edges(oracle, shape, bg, sp):
     assert np.array_equal(got, oracle.compose_hv(g, u, sp, 1, bg))
 
 
+@pytest.mark.parametrize("sp", [(1.0, 1.2, 1.0), (1.5, 0.75, 1.25), (1.2, 0.9, 2.06452), (2.0, 0.5, 1.0)])
+@pytest.mark.parametrize("shape", [(2, 2, 2), (3, 5, 129), (6, 2, 40)])
+@pytest.mark.parametrize("wrap", [False, True])
+def test_gradient_kernels_at_the_borders(oracle, sp, shape, wrap):
+    """Float and other spacings, one-sided and wrapped differences, axes of two voxels. Bit-exact."""
+    rng = np.random.default_rng(46)
+    img = rng.normal(0, 1, shape).astype(np.float32)
+    assert np.array_equal(host(D.gradient(cu(img), sp, wrap)), oracle.gradient(img, sp, wrap))
+
+
 @pytest.mark.parametrize("sp", [(1.5, 0.75, 1.25), (1.2, 0.9, 2.06452), (2.0, 0.5, 1.0)])
 def test_gradient_divisors(oracle, sp):
     """Spacings divided in float (exactly floats), in double, and multiplied."""
