@@ -83,6 +83,13 @@ cudaError_t launch_early(void (*kernel)(P...), dim3 grid, unsigned threads, size
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// the outcome of a launch_early, without leaving it behind for the next
+// caller of cudaGetLastError
+inline cudaError_t launched(cudaError_t e) {
+  const cudaError_t last = cudaGetLastError();
+  return e != cudaSuccess ? e : last;
+}
+
 // n / d for 0 <= n < 2^31 by multiply and shift (round-up method)
 struct IdxDiv {
   uint32_t d, mul, l;

@@ -1058,29 +1058,31 @@ template <class Src>
 cudaError_t any_forward(const AnyPlan &p, const Src &src, bool split, cudaStream_t s) {
   const AnyXY &a = p.xy;
   if (!split)
-    return launch_early(k_any_xy_fwd<Src>, dim3(a.d.nz, 3), p.threads_xy, p.smem_xy, s, a, src);
+    return launched(
+        launch_early(k_any_xy_fwd<Src>, dim3(a.d.nz, 3), p.threads_xy, p.smem_xy, s, a, src));
   const cudaError_t e = launch_early(k_any_x_fwd<Src>, dim3(a.d.nz, 3, (a.H + a.P - 1) / a.P), 256,
                                      p.smem_x, s, a, src);
-  if (e != cudaSuccess) return e;
-  return launch_early(k_any_y<-1>, dim3(a.d.nz, 3, (a.ncol + a.Q - 1) / a.Q), p.threads_y, p.smem_y,
-                      s, a);
+  if (e != cudaSuccess) return launched(e);
+  return launched(launch_early(k_any_y<-1>, dim3(a.d.nz, 3, (a.ncol + a.Q - 1) / a.Q), p.threads_y,
+                               p.smem_y, s, a));
 }
 
 template <class Dst>
 cudaError_t any_inverse(const AnyPlan &p, const Dst &dst, bool split, cudaStream_t s) {
   const AnyXY &a = p.xy;
   if (!split)
-    return launch_early(k_any_xy_inv<Dst>, dim3(a.d.nz, 3), p.threads_xy, p.smem_xy, s, a, dst);
+    return launched(
+        launch_early(k_any_xy_inv<Dst>, dim3(a.d.nz, 3), p.threads_xy, p.smem_xy, s, a, dst));
   const cudaError_t e = launch_early(k_any_y<+1>, dim3(a.d.nz, 3, (a.ncol + a.Q - 1) / a.Q),
                                      p.threads_y, p.smem_y, s, a);
-  if (e != cudaSuccess) return e;
-  return launch_early(k_any_x_inv<Dst>, dim3(a.d.nz, 3, (a.H + a.P - 1) / a.P), 256, p.smem_x, s, a,
-                      dst);
+  if (e != cudaSuccess) return launched(e);
+  return launched(launch_early(k_any_x_inv<Dst>, dim3(a.d.nz, 3, (a.H + a.P - 1) / a.P), 256, p.smem_x,
+                               s, a, dst));
 }
 
 cudaError_t any_solve(const AnyPlan &p, int inverse, cudaStream_t s) {
   const int grid = (int)((p.z.pcols + p.z.q - 1) / p.z.q);
-  return launch_early(k_any_z, dim3(grid), p.threads_z, p.smem_z, s, p.z, inverse);
+  return launched(launch_early(k_any_z, dim3(grid), p.threads_z, p.smem_z, s, p.z, inverse));
 }
 
 // the kernels of a plan and the shared memory each needs

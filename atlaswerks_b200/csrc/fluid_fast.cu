@@ -656,7 +656,7 @@ cudaError_t fast_xy_forward(const FluidPlan &p, const Src &src, cudaStream_t s) 
                        src);
     });
   });
-  return e;
+  return launched(e);
 }
 
 template <class Dst>
@@ -669,7 +669,7 @@ cudaError_t fast_xy_inverse(const FluidPlan &p, const Dst &dst, cudaStream_t s) 
                        dst);
     });
   });
-  return e;
+  return launched(e);
 }
 
 cudaError_t fast_xy_inverse_compose(const FluidPlan &p, const ComposeArgs &a, cudaStream_t s) {
@@ -706,7 +706,7 @@ cudaError_t fast_z_solve(const FluidPlan &p, int inverse, cudaStream_t s) {
     else
       go(k_z_solve_fast<NZ, 16, false>, z_threads<NZ, 16>());
   });
-  return e;
+  return launched(e);
 }
 
 template cudaError_t fast_xy_forward<SrcField>(const FluidPlan &, const SrcField &, cudaStream_t);

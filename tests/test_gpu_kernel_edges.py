@@ -168,6 +168,34 @@ def test_splat_scan_sizes(oracle, shape):
     assert np.array_equal(host(D.splat(cu(img), cu(h), 0.0)), oracle.splat(img, h, 0.0))
 
 
+@pytest.mark.parametrize("shape", [(12, 11, 10), (16, 32, 16)])
+def test_a_failed_launch_is_reported_once(shape):
+    """An operator called on a stream whose capture was given up reports that; a call on another stream does not."""
+    import ctypes
+    op = DiffOperB200()
+    op.SetSize(shape[::-1], (1.0, 1.0, 1.0), DiffOperParam())
+    v = torch.zeros((3,) + shape, device="cuda")
+    img, g = torch.rand(shape, device="cuda"), torch.zeros((3,) + shape, device="cuda")
+    L, rt = _lib.lib(), ctypes.CDLL("libcudart.so.12")
+    s = torch.cuda.Stream()
+    st = ctypes.c_void_p(s.cuda_stream)
+    torch.cuda.synchronize()
+    nz, ny, nx = shape
+    assert rt.cudaStreamBeginCapture(st, 2) == 0  # relaxed: other streams go on
+    try:
+        assert rt.cudaStreamSynchronize(st) != 0  # not allowed in a capture, which ends it
+        rt.cudaGetLastError()
+        assert L.aw_fluid_apply(op._h, *[t.data_ptr() for t in v], 1, st) != 0
+        rc = L.aw_gradient(img.data_ptr(), *[t.data_ptr() for t in g], nx, ny, nz, 1.0, 1.0, 1.0, 0, None)
+        msg = L.aw_last_error()
+    finally:
+        graph = ctypes.c_void_p()
+        rt.cudaStreamEndCapture(st, ctypes.byref(graph))
+        rt.cudaGetLastError()
+    assert rc == 0, msg
+    assert np.isfinite(host(op.ApplyInverseOperator(v))).all()
+
+
 def test_adjoint_shooting_memory():
     """The T + 1 kept sorts share one buffer of products: a handle at 80 x 96 x 112 with T = 5 stays below the
     fields' and the sorts' own memory plus one such buffer, which T + 2 of them would exceed by 90 MB."""
